@@ -118,132 +118,181 @@ __device__ inline void transport3(const qq::Su3<float>& u, bool back, float fac,
   }
 }
 
-// out = layer(w) in; w: [9][COUT][CIN] complex.
+// Component a of (T_p f)(x) for one channel: row a of the path's matrix (U forward, U^+
+// backward) times v, and the boundary factor.
+__device__ inline float2 transport_row(const qq::Su3<float>& u, bool back, int a, float fac, const float2* v) {
+  float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int b = 0; b < 3; ++b) {
+    const qq::cplx<float> e = a == 0 ? (back ? u.e[b][0] : u.e[0][b])
+                              : a == 1 ? (back ? u.e[b][1] : u.e[1][b]) : (back ? u.e[b][2] : u.e[2][b]);
+    cmacf(s, make_float2(e.re, back ? -e.im : e.im), v[b]);
+  }
+  return make_float2(fac * s.x, fac * s.y);
+}
+
+constexpr int kPtcSites = 64;
+
+// out = layer(w) in for one pair per blockIdx.y; w: [9][COUT][CIN] complex.
+// Bound by the FP32 multiply-adds of the channel mixing; a thread takes one colour of one
+// site, so a layer has three threads per site: enough warps on the small lattices, and no
+// work is repeated but the link's reconstruction.  The weights of one (path, input
+// channel) are read as COUT / 2 16-byte broadcasts.  (With a thread per site an 8 -> 8
+// layer of one pair on 8^3x16 had 64 blocks and took 30 us.  Twenty training steps on two
+// pairs there, 4-8-8-4: 42.2 -> 11.2 ms with this kernel, the weight gradient below and
+// the pairs of a group in one launch.)
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(kNetThreads) ptc_kernel(NetGeom g, const void* gauge, const float2* __restrict__ in,
-                                                          float2* __restrict__ out, const float2* __restrict__ w) {
-  __shared__ float2 sw[9 * COUT * CIN];
-  for (int i = threadIdx.x; i < 9 * COUT * CIN; i += blockDim.x) sw[i] = w[i];
+__global__ void __launch_bounds__(kPtcSites * 3) ptc_kernel(NetGeom g, const void* gauge, const float2* __restrict__ in,
+                                                            float2* __restrict__ out, const float2* __restrict__ w) {
+  __shared__ float4 sw[9 * CIN * COUT / 2];  // [path][ci][co]
+  for (int i = threadIdx.y * kPtcSites + threadIdx.x; i < 9 * COUT * CIN; i += 3 * kPtcSites) {
+    const int ci = i % CIN, co = (i / CIN) % COUT, p = i / (CIN * COUT);
+    reinterpret_cast<float2*>(sw)[(p * CIN + ci) * COUT + co] = w[i];
+  }
   __syncthreads();
-  const int L = blockIdx.x * blockDim.x + threadIdx.x;
+  const int L = blockIdx.x * kPtcSites + threadIdx.x, a = threadIdx.y;
   if (L >= g.V) return;
+  in += (size_t)blockIdx.y * CIN * 3 * g.V;
+  out += (size_t)blockIdx.y * COUT * 3 * g.V;
   int x[4];
   lex_coords(g, L, x);
-  float2 acc[COUT][3];
+  float2 acc[COUT];
 #pragma unroll
-  for (int co = 0; co < COUT; ++co)
-#pragma unroll
-    for (int a = 0; a < 3; ++a) acc[co][a] = make_float2(0.f, 0.f);
+  for (int co = 0; co < COUT; ++co) acc[co] = make_float2(0.f, 0.f);
   for (int p = 0; p < 9; ++p) {
     const PathSrc ps = path_src(g, x, L, p);
     if (ps.fac == 0.0f) continue;
     qq::Su3<float> u;
     if (p > 0) path_link(g, gauge, x, ps, u);
+#pragma unroll 4
     for (int ci = 0; ci < CIN; ++ci) {
+      float2 t;
+      if (p == 0) {
+        t = in[(size_t)(ci * 3 + a) * g.V + L];
+      } else {
+        float2 v[3];
+#pragma unroll
+        for (int b = 0; b < 3; ++b) v[b] = in[(size_t)(ci * 3 + b) * g.V + ps.L];
+        t = transport_row(u, ps.back, a, ps.fac, v);
+      }
+#pragma unroll
+      for (int co = 0; co < COUT; co += 2) {
+        const float4 wc = sw[((p * CIN + ci) * COUT + co) / 2];
+        cmacf(acc[co], make_float2(wc.x, wc.y), t);
+        cmacf(acc[co + 1], make_float2(wc.z, wc.w), t);
+      }
+    }
+  }
+#pragma unroll
+  for (int co = 0; co < COUT; ++co) out[(size_t)(co * 3 + a) * g.V + L] = acc[co];
+}
+
+// grad[p][co][ci] = sum_x sum_a delta_co(x)_a conj((T_p f_ci)(x)_a), in FP64, as one
+// partial per block of the grid's x: partial[(block * 9 + p) * COUT * CIN + co * CIN + ci].
+// A block takes one path (blockIdx.y) and every gridDim.x-th chunk of sites of all pairs.
+// It transports a chunk's fields once into shared memory, as doubles, and multiplies them
+// there as a (COUT x rows) by (rows x CIN) product with a 2 x 2 tile per thread: the
+// threads left over by the tile count share the rows, and meet once at the end.  Bound by
+// shared-memory reads (four 16-byte reads for 16 FP64 multiply-adds); a block-wide
+// reduction per (path, input channel) took 87 us for 8 -> 8 on 8^3x16.
+template <int CIN, int COUT>
+__global__ void __launch_bounds__(kNetThreads) ptc_wgrad_kernel(NetGeom g, const void* gauge, int pairs,
+                                                                const float2* __restrict__ delta,
+                                                                const float2* __restrict__ fin, double2* partial) {
+  constexpr int SC = CIN + COUT <= 16 ? 32 : 16;          // sites of a chunk
+  constexpr int NT = (COUT / 2) * (CIN / 2);              // tiles of a row slice
+  constexpr int NS = kNetThreads / NT, PER = kNetThreads / SC;
+  constexpr int kRows = 3 * SC;
+  constexpr int kShared = kRows * (COUT + CIN) > kNetThreads * 4 ? kRows * (COUT + CIN) : kNetThreads * 4;
+  __shared__ double2 sm[kShared];
+  double2* sd = sm;                  // [row][COUT]
+  double2* st = sm + kRows * COUT;   // [row][CIN]
+  const int p = blockIdx.y, tid = threadIdx.x, site = tid % SC, grp = tid / SC;
+  const int tile = tid % NT, slice = tid / NT, m = 2 * (tile / (CIN / 2)), n = 2 * (tile % (CIN / 2));
+  double2 acc[2][2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) acc[i][j] = make_double2(0.0, 0.0);
+  const int chunks = g.V / SC;  // the volume is a multiple of 256
+  for (int unit = blockIdx.x; unit < pairs * chunks; unit += gridDim.x) {
+    const int pair = unit / chunks, L = (unit % chunks) * SC + site;
+    int x[4];
+    lex_coords(g, L, x);
+    const PathSrc ps = path_src(g, x, L, p);
+    qq::Su3<float> u;
+    if (p > 0 && ps.fac != 0.0f) path_link(g, gauge, x, ps, u);
+    const float2* f = fin + (size_t)pair * CIN * 3 * g.V + ps.L;
+    for (int ci = grp; ci < CIN; ci += PER) {
       float2 v[3], t[3];
 #pragma unroll
-      for (int a = 0; a < 3; ++a) v[a] = in[(size_t)(ci * 3 + a) * g.V + ps.L];
+      for (int a = 0; a < 3; ++a) v[a] = f[(size_t)(ci * 3 + a) * g.V];
       if (p == 0) {
 #pragma unroll
         for (int a = 0; a < 3; ++a) t[a] = v[a];
-      } else {
+      } else if (ps.fac != 0.0f) {
         transport3(u, ps.back, ps.fac, v, t);
+      } else {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) t[a] = make_float2(0.f, 0.f);
       }
 #pragma unroll
-      for (int co = 0; co < COUT; ++co) {
-        const float2 wc = sw[(p * COUT + co) * CIN + ci];
-#pragma unroll
-        for (int a = 0; a < 3; ++a) cmacf(acc[co][a], wc, t[a]);
-      }
+      for (int a = 0; a < 3; ++a) st[(a * SC + site) * CIN + ci] = make_double2((double)t[a].x, (double)t[a].y);
     }
+    const float2* d = delta + (size_t)pair * COUT * 3 * g.V + L;
+    for (int co = grp; co < COUT; co += PER)
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        const float2 v = d[(size_t)(co * 3 + a) * g.V];
+        sd[(a * SC + site) * COUT + co] = make_double2((double)v.x, (double)v.y);
+      }
+    __syncthreads();
+    for (int r = slice; r < kRows; r += NS) {
+      const double2 d0 = sd[r * COUT + m], d1 = sd[r * COUT + m + 1];
+      const double2 t0 = st[r * CIN + n], t1 = st[r * CIN + n + 1];
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const double2 dd = i ? d1 : d0, tt = j ? t1 : t0;  // d conj(t)
+          acc[i][j].x += dd.x * tt.x + dd.y * tt.y;
+          acc[i][j].y += dd.y * tt.x - dd.x * tt.y;
+        }
+    }
+    __syncthreads();
   }
 #pragma unroll
-  for (int co = 0; co < COUT; ++co)
+  for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int a = 0; a < 3; ++a) out[(size_t)(co * 3 + a) * g.V + L] = acc[co][a];
-}
-
-// Per-block partial of grad[p][co][ci] = sum_x sum_a delta_co(x)_a conj((T_p f_ci)(x)_a),
-// in FP64: partial[(block * 9 * COUT + p * COUT + co) * CIN + ci] (complex).
-template <int CIN, int COUT>
-__global__ void __launch_bounds__(kNetThreads) ptc_wgrad_kernel(NetGeom g, const void* gauge,
-                                                                const float2* __restrict__ delta,
-                                                                const float2* __restrict__ fin, double2* partial) {
-  __shared__ double2 red[kNetThreads / 32][COUT];
-  const int L = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool act = L < g.V;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int x[4] = {0, 0, 0, 0};
-  if (act) lex_coords(g, L, x);
-  float2 d[COUT][3];
-#pragma unroll
-  for (int co = 0; co < COUT; ++co)
-#pragma unroll
-    for (int a = 0; a < 3; ++a) d[co][a] = act ? delta[(size_t)(co * 3 + a) * g.V + L] : make_float2(0.f, 0.f);
-  for (int p = 0; p < 9; ++p) {
-    PathSrc ps{L, 0.0f, 0, 0};
-    qq::Su3<float> u;
-    if (act) {
-      ps = path_src(g, x, L, p);
-      if (p > 0 && ps.fac != 0.0f) path_link(g, gauge, x, ps, u);
+    for (int j = 0; j < 2; ++j) sm[(size_t)slice * COUT * CIN + (m + i) * CIN + n + j] = acc[i][j];
+  __syncthreads();
+  for (int e = tid; e < COUT * CIN; e += kNetThreads) {
+    double2 s = sm[e];
+    for (int k = 1; k < NS; ++k) {
+      s.x += sm[k * COUT * CIN + e].x;
+      s.y += sm[k * COUT * CIN + e].y;
     }
-    for (int ci = 0; ci < CIN; ++ci) {
-      float2 t[3] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-      if (act && ps.fac != 0.0f) {
-        float2 v[3];
-#pragma unroll
-        for (int a = 0; a < 3; ++a) v[a] = fin[(size_t)(ci * 3 + a) * g.V + ps.L];
-        if (p == 0) {
-#pragma unroll
-          for (int a = 0; a < 3; ++a) t[a] = v[a];
-        } else {
-          transport3(u, ps.back, ps.fac, v, t);
-        }
-      }
-#pragma unroll
-      for (int co = 0; co < COUT; ++co) {
-        double re = 0.0, im = 0.0;
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {  // d conj(t)
-          re += (double)d[co][a].x * t[a].x + (double)d[co][a].y * t[a].y;
-          im += (double)d[co][a].y * t[a].x - (double)d[co][a].x * t[a].y;
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          re += __shfl_down_sync(0xffffffffu, re, o);
-          im += __shfl_down_sync(0xffffffffu, im, o);
-        }
-        if (lane == 0) red[warp][co] = make_double2(re, im);
-      }
-      __syncthreads();
-      if (threadIdx.x < COUT) {
-        double2 s = red[0][threadIdx.x];
-        for (int wi = 1; wi < kNetThreads / 32; ++wi) {
-          s.x += red[wi][threadIdx.x].x;
-          s.y += red[wi][threadIdx.x].y;
-        }
-        partial[((size_t)blockIdx.x * 9 * COUT + (size_t)p * COUT + threadIdx.x) * CIN + ci] = s;
-      }
-      __syncthreads();
-    }
+    partial[((size_t)blockIdx.x * 9 + p) * COUT * CIN + e] = s;
   }
 }
 
-// grad[e] (+)= sum over blocks of partial[block][e], fixed order.
-__global__ void net_grad_sum_kernel(const double2* partial, int nblocks, int ne, double2* grad, int accumulate) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+// grad[e] += sum over blocks of partial[block][e]: a warp per entry, fixed order.
+__global__ void __launch_bounds__(kNetThreads) net_grad_sum_kernel(const double2* partial, int nblocks, int ne,
+                                                                   double2* grad) {
+  const int e = (blockIdx.x * kNetThreads + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (e >= ne) return;
   double2 s = make_double2(0.0, 0.0);
-  for (int b = 0; b < nblocks; ++b) {
+  for (int b = lane; b < nblocks; b += 32) {
     const double2 v = partial[(size_t)b * ne + e];
     s.x += v.x;
     s.y += v.y;
   }
-  if (accumulate) {
-    s.x += grad[e].x;
-    s.y += grad[e].y;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    s.x += __shfl_down_sync(0xffffffffu, s.x, o);
+    s.y += __shfl_down_sync(0xffffffffu, s.y, o);
   }
-  grad[e] = s;
+  if (lane == 0) grad[e] = make_double2(grad[e].x + s.x, grad[e].y + s.y);
 }
 
 // even-site FP64 spinor (checkerboard index) -> 4-channel net field (odd sites untouched)
@@ -275,12 +324,18 @@ __global__ void net_extract_kernel(qq::Geom gg, NetGeom g, const float2* in, qq:
   qq::SpinorIO<qq::P64>::store(out.data, out.norm, gg.vh, s, v);
 }
 
-// delta = scale (out - target) on even sites, 0 on odd; partial[block] = sum |out - target|^2
-// over even sites (FP64).
+// For pair blockIdx.y: delta = scale (out - target) on even sites, 0 on odd;
+// partial[pair * blocks + block] = sum |out - target|^2 over even sites (FP64).
 __global__ void __launch_bounds__(kNetThreads) net_residual_kernel(NetGeom g, const float2* out, const float2* target,
-                                                                   float2* delta, double scale, double* partial) {
+                                                                   float2* delta, const double* scales,
+                                                                   double* partial) {
   __shared__ double red[kNetThreads / 32];
   const int L = blockIdx.x * blockDim.x + threadIdx.x;
+  const double scale = scales[blockIdx.y];
+  const size_t pair = (size_t)blockIdx.y * 12 * g.V;
+  out += pair;
+  target += pair;
+  delta += pair;
   double s = 0.0;
   if (L < g.V) {
     int x[4];
@@ -304,7 +359,7 @@ __global__ void __launch_bounds__(kNetThreads) net_residual_kernel(NetGeom g, co
   if (threadIdx.x == 0) {
     double t = 0.0;
     for (int wi = 0; wi < kNetThreads / 32; ++wi) t += red[wi];
-    partial[blockIdx.x] = t;
+    partial[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = t;
   }
 }
 
@@ -331,16 +386,22 @@ __global__ void net_gauss_kernel(int vh, unsigned long long seed, qq::Spinor out
 }
 
 template <int CIN, int COUT>
-cudaError_t launch_ptc(const NetGeom& g, const void* gauge, const float2* in, float2* out, const float2* w,
+cudaError_t launch_ptc(const NetGeom& g, const void* gauge, int pairs, const float2* in, float2* out, const float2* w,
                        cudaStream_t st) {
-  ptc_kernel<CIN, COUT><<<(g.V + kNetThreads - 1) / kNetThreads, kNetThreads, 0, st>>>(g, gauge, in, out, w);
+  ptc_kernel<CIN, COUT><<<dim3((g.V + kPtcSites - 1) / kPtcSites, pairs), dim3(kPtcSites, 3), 0, st>>>(g, gauge, in, out,
+                                                                                                     w);
   return cudaGetLastError();
 }
+// Partials of a weight gradient: about four blocks per SM over the nine paths, and no more
+// than there are chunks of sites.
+constexpr int kWgradBlocks = 64;
+inline int wgrad_blocks(const NetGeom& g, int pairs) { return std::min(kWgradBlocks, pairs * (g.V / 32)); }
+
 template <int CIN, int COUT>
-cudaError_t launch_wgrad(const NetGeom& g, const void* gauge, const float2* delta, const float2* fin, double2* part,
-                         cudaStream_t st) {
-  ptc_wgrad_kernel<CIN, COUT><<<(g.V + kNetThreads - 1) / kNetThreads, kNetThreads, 0, st>>>(g, gauge, delta, fin,
-                                                                                              part);
+cudaError_t launch_wgrad(const NetGeom& g, const void* gauge, int pairs, const float2* delta, const float2* fin,
+                         double2* part, cudaStream_t st) {
+  ptc_wgrad_kernel<CIN, COUT><<<dim3(wgrad_blocks(g, pairs), 9), kNetThreads, 0, st>>>(g, gauge, pairs, delta, fin,
+                                                                                       part);
   return cudaGetLastError();
 }
 
@@ -358,15 +419,15 @@ cudaError_t launch_wgrad(const NetGeom& g, const void* gauge, const float2* delt
     default: return cudaErrorInvalidValue;                                      \
   }
 
-cudaError_t ptc(int ci, int co, const NetGeom& g, const void* gauge, const float2* in, float2* out, const float2* w,
-                cudaStream_t st) {
+cudaError_t ptc(int ci, int co, const NetGeom& g, const void* gauge, int pairs, const float2* in, float2* out,
+                const float2* w, cudaStream_t st) {
   qq::count_launch();
-  QQ_NET_DISPATCH(launch_ptc, ci, co, g, gauge, in, out, w, st)
+  QQ_NET_DISPATCH(launch_ptc, ci, co, g, gauge, pairs, in, out, w, st)
 }
-cudaError_t wgrad(int ci, int co, const NetGeom& g, const void* gauge, const float2* delta, const float2* fin,
+cudaError_t wgrad(int ci, int co, const NetGeom& g, const void* gauge, int pairs, const float2* delta, const float2* fin,
                   double2* part, cudaStream_t st) {
   qq::count_launch();
-  QQ_NET_DISPATCH(launch_wgrad, ci, co, g, gauge, delta, fin, part, st)
+  QQ_NET_DISPATCH(launch_wgrad, ci, co, g, gauge, pairs, delta, fin, part, st)
 }
 
 }  // namespace qqnet
@@ -381,13 +442,16 @@ struct qq_net {
   int ch[kNetMaxLayers + 1] = {};
   std::vector<std::complex<double>> w;  // [layer][9][co][ci], FP64 master copy
   std::vector<size_t> off;              // first weight of each layer
-  DevBuf wf, wa;                        // FP32 weights and adjoint weights on the device
+  DevBuf wf;                            // FP32 weights, then adjoint weights, on the device
+  std::vector<float2> wh;               // the same on the host (source of the upload)
   DevBuf acts[kNetMaxLayers + 1];       // activations (acts[0]: the embedded input), kept
-  int wdev = -1;                        // device of wf / wa / acts
+  int wdev = -1;                        // device of wf / acts
   bool dirty = true;
   std::vector<double> am, av;           // Adam moments (real, imaginary interleaved)
   int at = 0;
   size_t nw() const { return w.size(); }
+  const float2* fwd(int l) const { return wf.as<float2>() + off[l]; }
+  const float2* adj(int l) const { return wf.as<float2>() + nw() + off[l]; }
 };
 
 namespace qq {
@@ -410,19 +474,22 @@ size_t net_field_bytes(qq_ctx* c, int channels) { return (size_t)channels * 3 * 
 // FP32 weights and adjoint weights of every layer on the context's device.
 int net_upload(qq_ctx* c, qq_net* net) {
   if (!net->dirty && net->wdev == c->device) return QQ_OK;
-  if (net->wdev != c->device)  // buffers of another device: release them
-    for (DevBuf& b : net->acts)
-      if (b.p) {
-        cudaFree(b.p);
-        b.p = nullptr;
-        b.bytes = 0;
-      }
-  std::vector<float2> wf(net->nw()), wa(net->nw());
+  if (net->wdev != c->device) {  // buffers of another device: release them
+    auto drop = [](DevBuf& b) {
+      if (b.p) cudaFree(b.p);
+      b.p = nullptr;
+      b.bytes = 0;
+    };
+    for (DevBuf& b : net->acts) drop(b);
+    drop(net->wf);
+  }
+  QQ_CK(cudaStreamSynchronize(c->st));  // an earlier upload has left wh
+  net->wh.resize(2 * net->nw());
   for (int l = 0; l < net->nl; ++l) {
     const int ci = net->ch[l], co = net->ch[l + 1];
     const std::complex<double>* W = net->w.data() + net->off[l];
-    float2* F = wf.data() + net->off[l];
-    float2* A = wa.data() + net->off[l];  // adjoint: [9][ci][co]
+    float2* F = net->wh.data() + net->off[l];
+    float2* A = net->wh.data() + net->nw() + net->off[l];  // adjoint: [9][ci][co]
     for (int p = 0; p < 9; ++p)
       for (int o = 0; o < co; ++o)
         for (int i = 0; i < ci; ++i) {
@@ -432,23 +499,21 @@ int net_upload(qq_ctx* c, qq_net* net) {
           A[((size_t)pa * ci + i) * co + o] = make_float2((float)v.real(), (float)-v.imag());
         }
   }
-  QQ_CK(net->wf.alloc(sizeof(float2) * wf.size()));
-  QQ_CK(net->wa.alloc(sizeof(float2) * wa.size()));
-  QQ_CK(cudaMemcpyAsync(net->wf.p, wf.data(), sizeof(float2) * wf.size(), cudaMemcpyHostToDevice, c->st));
-  QQ_CK(cudaMemcpyAsync(net->wa.p, wa.data(), sizeof(float2) * wa.size(), cudaMemcpyHostToDevice, c->st));
-  QQ_CK(cudaStreamSynchronize(c->st));
+  QQ_CK(net->wf.alloc(sizeof(float2) * net->wh.size()));
+  QQ_CK(cudaMemcpyAsync(net->wf.p, net->wh.data(), sizeof(float2) * net->wh.size(), cudaMemcpyHostToDevice, c->st));
   net->wdev = c->device;
   net->dirty = false;
   return QQ_OK;
 }
 
-// acts[l + 1] = layer l applied to (l == 0 ? input : acts[l]); acts[0] is not used.
-int net_forward(qq_ctx* c, qq_net* net, const float2* input, DevBuf* acts) {
+// acts[l + 1] = layer l applied to (l == 0 ? input : acts[l]), `pairs` fields one after
+// another; acts[0] is not used.
+int net_forward(qq_ctx* c, qq_net* net, int pairs, const float2* input, DevBuf* acts) {
   const NetGeom g = net_geom(c);
   for (int l = 0; l < net->nl; ++l) {
-    QQ_CK(acts[l + 1].alloc(net_field_bytes(c, net->ch[l + 1])));
-    QQ_CK(ptc(net->ch[l], net->ch[l + 1], g, c->gauge32.p, l == 0 ? input : acts[l].as<float2>(),
-              acts[l + 1].as<float2>(), net->wf.as<float2>() + net->off[l], c->st));
+    QQ_CK(acts[l + 1].alloc(net_field_bytes(c, net->ch[l + 1]) * pairs));
+    QQ_CK(ptc(net->ch[l], net->ch[l + 1], g, c->gauge32.p, pairs, l == 0 ? input : acts[l].as<float2>(),
+              acts[l + 1].as<float2>(), net->fwd(l), c->st));
   }
   return QQ_OK;
 }
@@ -468,7 +533,7 @@ int net_apply_field(qq_ctx* c, qq_net* net, Spinor out, Spinor in) {
   count_launch(2);
   net_embed_kernel<<<nblk, 128, 0, c->st>>>(c->g, g, in, acts[0].as<float2>());
   QQ_CK(cudaGetLastError());
-  QQ_TRY(net_forward(c, net, acts[0].as<float2>(), acts));
+  QQ_TRY(net_forward(c, net, 1, acts[0].as<float2>(), acts));
   net_extract_kernel<<<nblk, 128, 0, c->st>>>(c->g, g, acts[net->nl].as<float2>(), out);
   QQ_CK(cudaGetLastError());
   return QQ_OK;
@@ -476,78 +541,103 @@ int net_apply_field(qq_ctx* c, qq_net* net, Spinor out, Spinor in) {
 
 namespace {
 
-// Loss and gradient (accumulated into grad, complex [nw]) over pairs of embedded net
-// fields B[i], X[i]; returns the loss.
-int net_loss_grad(qq_ctx* c, qq_net* net, const std::vector<DevBuf>& B, const std::vector<DevBuf>& X,
-                  const std::vector<double>& xnorm2, DevBuf& grad, double* loss) {
+// Device buffers of a training call, kept over its steps.
+struct NetScratch {
+  DevBuf part, lpart, scale, d0, d1, grad;
+};
+
+// Pairs that go through the layers together: up to 8, within 512 MiB of activations (at
+// least one), so that small lattices fill the GPU and large ones need no more memory.
+int net_group(qq_ctx* c, const qq_net* net, int pairs) {
+  size_t bytes = 0;
+  for (int l = 0; l <= net->nl; ++l) bytes += net_field_bytes(c, net->ch[l]);
+  const size_t fit = std::max<size_t>(1, ((size_t)512 << 20) / bytes);
+  return (int)std::min<size_t>({fit, (size_t)8, (size_t)pairs});
+}
+
+// Loss and gradient (scratch.grad, complex [nw]) over S pairs of embedded net fields, one
+// after another in B and X; grad_host receives the gradient.
+int net_loss_grad(qq_ctx* c, qq_net* net, int S, const DevBuf& B, const DevBuf& X, const std::vector<double>& xnorm2,
+                  NetScratch& N, std::vector<double2>& grad_host, double* loss) {
   QQ_TRY(net_upload(c, net));
   const NetGeom g = net_geom(c);
-  const int S = (int)B.size();
-  const int nblk = (g.V + kNetThreads - 1) / kNetThreads;
+  const int nblk = (g.V + kNetThreads - 1) / kNetThreads, group = net_group(c, net, S);
+  const size_t field = (size_t)12 * g.V;
   int maxc = 4;
   for (int l = 0; l <= net->nl; ++l) maxc = std::max(maxc, net->ch[l]);
-  DevBuf part, lpart, d0, d1;
-  QQ_CK(part.alloc(sizeof(double2) * (size_t)nblk * 9 * maxc * maxc));
-  QQ_CK(lpart.alloc(sizeof(double) * nblk));
-  QQ_CK(d0.alloc(net_field_bytes(c, maxc)));
-  QQ_CK(d1.alloc(net_field_bytes(c, maxc)));
-  QQ_CK(grad.alloc(sizeof(double2) * net->nw()));
-  QQ_CK(cudaMemsetAsync(grad.p, 0, grad.bytes, c->st));
-  std::vector<double> lp(nblk);
-  DevBuf* acts = net->acts;
-  double total = 0.0;
-  for (int i = 0; i < S; ++i) {
-    QQ_TRY(net_forward(c, net, B[i].as<float2>(), acts));
-    const double scale = 1.0 / ((double)S * xnorm2[i]);
-    count_launch();
-    net_residual_kernel<<<nblk, kNetThreads, 0, c->st>>>(g, acts[net->nl].as<float2>(), X[i].as<float2>(),
-                                                         d0.as<float2>(), scale, lpart.as<double>());
-    QQ_CK(cudaGetLastError());
-    QQ_CK(cudaMemcpyAsync(lp.data(), lpart.p, sizeof(double) * nblk, cudaMemcpyDeviceToHost, c->st));
+  QQ_CK(N.part.alloc(sizeof(double2) * (size_t)kWgradBlocks * 9 * maxc * maxc));
+  QQ_CK(N.lpart.alloc(sizeof(double) * nblk * (size_t)S));
+  QQ_CK(N.d0.alloc(net_field_bytes(c, maxc) * group));
+  QQ_CK(N.d1.alloc(net_field_bytes(c, maxc) * group));
+  QQ_CK(N.grad.alloc(sizeof(double2) * net->nw()));
+  QQ_CK(cudaMemsetAsync(N.grad.p, 0, sizeof(double2) * net->nw(), c->st));
+  if (!N.scale.p) {
+    std::vector<double> sc(S);
+    for (int i = 0; i < S; ++i) sc[i] = 1.0 / ((double)S * xnorm2[i]);
+    QQ_CK(N.scale.alloc(sizeof(double) * S));
+    QQ_CK(cudaMemcpyAsync(N.scale.p, sc.data(), sizeof(double) * S, cudaMemcpyHostToDevice, c->st));
     QQ_CK(cudaStreamSynchronize(c->st));
-    double li = 0.0;
-    for (double v : lp) li += v;
-    total += li / ((double)S * xnorm2[i]);
-    DevBuf* dcur = &d0;
-    DevBuf* dnext = &d1;
+  }
+  DevBuf* acts = net->acts;
+  for (int i = 0; i < S; i += group) {
+    const int np = std::min(group, S - i);
+    const float2* in = B.as<float2>() + i * field;
+    QQ_TRY(net_forward(c, net, np, in, acts));
+    count_launch();
+    net_residual_kernel<<<dim3(nblk, np), kNetThreads, 0, c->st>>>(g, acts[net->nl].as<float2>(),
+                                                                   X.as<float2>() + i * field, N.d0.as<float2>(),
+                                                                   N.scale.as<double>() + i,
+                                                                   N.lpart.as<double>() + (size_t)i * nblk);
+    QQ_CK(cudaGetLastError());
+    DevBuf* dcur = &N.d0;
+    DevBuf* dnext = &N.d1;
     for (int l = net->nl - 1; l >= 0; --l) {
       const int ci = net->ch[l], co = net->ch[l + 1];
       const int ne = 9 * co * ci;
-      const float2* fin = l == 0 ? B[i].as<float2>() : acts[l].as<float2>();
-      QQ_CK(wgrad(ci, co, g, c->gauge32.p, dcur->as<float2>(), fin, part.as<double2>(), c->st));
+      const float2* fin = l == 0 ? in : acts[l].as<float2>();
+      QQ_CK(wgrad(ci, co, g, c->gauge32.p, np, dcur->as<float2>(), fin, N.part.as<double2>(), c->st));
       count_launch();
-      net_grad_sum_kernel<<<(ne + 127) / 128, 128, 0, c->st>>>(part.as<double2>(), nblk, ne,
-                                                              grad.as<double2>() + net->off[l], 1);
+      net_grad_sum_kernel<<<(ne * 32 + kNetThreads - 1) / kNetThreads, kNetThreads, 0, c->st>>>(
+          N.part.as<double2>(), wgrad_blocks(g, np), ne, N.grad.as<double2>() + net->off[l]);
       QQ_CK(cudaGetLastError());
       if (l > 0) {
-        QQ_CK(ptc(co, ci, g, c->gauge32.p, dcur->as<float2>(), dnext->as<float2>(), net->wa.as<float2>() + net->off[l],
-                  c->st));
+        QQ_CK(ptc(co, ci, g, c->gauge32.p, np, dcur->as<float2>(), dnext->as<float2>(), net->adj(l), c->st));
         std::swap(dcur, dnext);
       }
     }
   }
+  std::vector<double> lp((size_t)nblk * S);
+  grad_host.resize(net->nw());
+  QQ_CK(cudaMemcpyAsync(lp.data(), N.lpart.p, sizeof(double) * lp.size(), cudaMemcpyDeviceToHost, c->st));
+  QQ_CK(cudaMemcpyAsync(grad_host.data(), N.grad.p, sizeof(double2) * net->nw(), cudaMemcpyDeviceToHost, c->st));
   QQ_CK(cudaStreamSynchronize(c->st));
+  double total = 0.0;
+  for (int i = 0; i < S; ++i) {
+    double li = 0.0;
+    for (int b = 0; b < nblk; ++b) li += lp[(size_t)i * nblk + b];
+    total += li / ((double)S * xnorm2[i]);
+  }
   *loss = total;
   return QQ_OK;
 }
 
-// Even-site reference half vectors -> embedded net fields (and |x|^2 of each); out
-// holds n buffers.
-int net_embed_refs(qq_ctx* c, int n, const double* refs, std::vector<DevBuf>& out, std::vector<double>* norm2) {
+// Even-site reference half vectors -> embedded net fields, one after another (and |x|^2
+// of each).
+int net_embed_refs(qq_ctx* c, int n, const double* refs, DevBuf& out, std::vector<double>* norm2) {
   const NetGeom g = net_geom(c);
   const size_t nv = c->ref_doubles();
   Tmp t(c, P64);
   if (norm2) norm2->resize(n);
   const int nblk = (c->g.vh + 127) / 128;
+  QQ_CK(out.alloc(net_field_bytes(c, 4) * n));
+  QQ_CK(cudaMemsetAsync(out.p, 0, net_field_bytes(c, 4) * n, c->st));
   for (int i = 0; i < n; ++i) {
     const double* d = nullptr;
     QQ_TRY(stage_in(c, 1, refs + (size_t)i * nv, nv, &d));
     QQ_TRY(ref_to_field(c, d, 0, t.sp()));
     if (norm2) QQ_TRY(norm2_host(c, t.sp(), &(*norm2)[i]));
-    QQ_CK(out[i].alloc(net_field_bytes(c, 4)));
-    QQ_CK(cudaMemsetAsync(out[i].p, 0, out[i].bytes, c->st));
     count_launch();
-    net_embed_kernel<<<nblk, 128, 0, c->st>>>(c->g, g, t.sp(), out[i].as<float2>());
+    net_embed_kernel<<<nblk, 128, 0, c->st>>>(c->g, g, t.sp(), out.as<float2>() + (size_t)i * 12 * g.V);
     QQ_CK(cudaGetLastError());
   }
   QQ_CK(cudaStreamSynchronize(c->st));
@@ -652,22 +742,23 @@ extern "C" int qq_net_grad(qq_ctx* c, qq_net* net, int nsamples, const double* b
                            double* grad) {
   QQ_TRY(net_check(c, net));
   if (nsamples < 1 || !b || !x || !loss || !grad) return set_error(QQ_BAD_ARG, "bad arguments");
-  std::vector<DevBuf> B(nsamples), X(nsamples);
+  DevBuf B, X;
   std::vector<double> xn2;
   QQ_TRY(net_embed_refs(c, nsamples, b, B, nullptr));
   QQ_TRY(net_embed_refs(c, nsamples, x, X, &xn2));
   for (double v : xn2)
     if (!(v > 0.0)) return set_error(QQ_BAD_ARG, "a target vector is zero");
-  DevBuf g;
-  QQ_TRY(net_loss_grad(c, net, B, X, xn2, g, loss));
-  QQ_CK(cudaMemcpy(grad, g.p, sizeof(double2) * net->nw(), cudaMemcpyDeviceToHost));
+  NetScratch N;
+  std::vector<double2> gh;
+  QQ_TRY(net_loss_grad(c, net, nsamples, B, X, xn2, N, gh, loss));
+  std::memcpy(grad, gh.data(), sizeof(double2) * net->nw());
   return QQ_OK;
 }
 
 namespace qq {
 namespace {
-int adam_steps(qq_ctx* c, qq_net* net, const std::vector<DevBuf>& B, const std::vector<DevBuf>& X,
-               const std::vector<double>& xn2, int nsteps, double lr, double* losses);
+int adam_steps(qq_ctx* c, qq_net* net, const DevBuf& B, const DevBuf& X, const std::vector<double>& xn2, int nsteps,
+               double lr, double* losses);
 }  // namespace
 }  // namespace qq
 
@@ -677,8 +768,13 @@ extern "C" int qq_net_train(qq_ctx* c, qq_net* net, const double kappa[2], int n
   if (!kappa || nsamples < 1 || nsteps < 0 || !(lr > 0.0)) return set_error(QQ_BAD_ARG, "bad arguments");
   // pairs (b = A x, x) with Gaussian x on the even sites
   const NetGeom g = net_geom(c);
-  std::vector<DevBuf> B(nsamples), X(nsamples);
+  DevBuf B, X;
   std::vector<double> xn2(nsamples);
+  const size_t field = (size_t)12 * g.V;
+  for (auto* pr : {&B, &X}) {
+    QQ_CK(pr->alloc(net_field_bytes(c, 4) * nsamples));
+    QQ_CK(cudaMemsetAsync(pr->p, 0, net_field_bytes(c, 4) * nsamples, c->st));
+  }
   Tmp xf(c, P64), bf(c, P64), tmp(c, P64);
   const int nblk = (c->g.vh + 127) / 128;
   for (int i = 0; i < nsamples; ++i) {
@@ -687,13 +783,9 @@ extern "C" int qq_net_train(qq_ctx* c, qq_net* net, const double kappa[2], int n
     QQ_CK(cudaGetLastError());
     QQ_TRY(op_dbletm(c, bf.sp(), xf.sp(), tmp.sp(), 0, kappa));
     QQ_TRY(norm2_host(c, xf.sp(), &xn2[i]));
-    for (auto* pr : {&B[i], &X[i]}) {
-      QQ_CK(pr->alloc(net_field_bytes(c, 4)));
-      QQ_CK(cudaMemsetAsync(pr->p, 0, pr->bytes, c->st));
-    }
     count_launch(2);
-    net_embed_kernel<<<nblk, 128, 0, c->st>>>(c->g, g, bf.sp(), B[i].as<float2>());
-    net_embed_kernel<<<nblk, 128, 0, c->st>>>(c->g, g, xf.sp(), X[i].as<float2>());
+    net_embed_kernel<<<nblk, 128, 0, c->st>>>(c->g, g, bf.sp(), B.as<float2>() + i * field);
+    net_embed_kernel<<<nblk, 128, 0, c->st>>>(c->g, g, xf.sp(), X.as<float2>() + i * field);
     QQ_CK(cudaGetLastError());
   }
   return adam_steps(c, net, B, X, xn2, nsteps, lr, losses);
@@ -703,7 +795,7 @@ extern "C" int qq_net_train_pairs(qq_ctx* c, qq_net* net, int nsamples, const do
                                   double lr, double* losses) {
   QQ_TRY(net_check(c, net));
   if (nsamples < 1 || !b || !x || nsteps < 0 || !(lr > 0.0)) return set_error(QQ_BAD_ARG, "bad arguments");
-  std::vector<DevBuf> B(nsamples), X(nsamples);
+  DevBuf B, X;
   std::vector<double> xn2;
   QQ_TRY(net_embed_refs(c, nsamples, b, B, nullptr));
   QQ_TRY(net_embed_refs(c, nsamples, x, X, &xn2));
@@ -716,18 +808,17 @@ namespace qq {
 namespace {
 // nsteps Adam steps (learning rate lr) on the loss of net_loss_grad over the embedded
 // pairs (B[i], X[i]); losses[step] (may be null) = the loss before each step.
-int adam_steps(qq_ctx* c, qq_net* net, const std::vector<DevBuf>& B, const std::vector<DevBuf>& X,
-               const std::vector<double>& xn2, int nsteps, double lr, double* losses) {
+int adam_steps(qq_ctx* c, qq_net* net, const DevBuf& B, const DevBuf& X, const std::vector<double>& xn2, int nsteps,
+               double lr, double* losses) {
   const size_t n = net->nw();
   std::vector<double2> gh(n);
+  NetScratch N;
   constexpr double b1 = 0.9, b2 = 0.999, eps = 1e-12;
   for (int step = 0; step < nsteps; ++step) {
-    DevBuf gd;
     double loss = 0.0;
-    QQ_TRY(net_loss_grad(c, net, B, X, xn2, gd, &loss));
+    QQ_TRY(net_loss_grad(c, net, (int)xn2.size(), B, X, xn2, N, gh, &loss));
     if (!std::isfinite(loss)) return set_error(QQ_NAN, "NaN loss in network training");
     if (losses) losses[step] = loss;
-    QQ_CK(cudaMemcpy(gh.data(), gd.p, sizeof(double2) * n, cudaMemcpyDeviceToHost));
     ++net->at;
     const double c1 = 1.0 - std::pow(b1, net->at), c2 = 1.0 - std::pow(b2, net->at);
     for (size_t i = 0; i < n; ++i) {
