@@ -52,8 +52,7 @@ struct qq_eig {
 
 namespace qq {
 
-int loop_slices(qq_ctx* c, const double* ye, const double* yo, const double* be, const double* bo, int ksub,
-                double* val, double* Jdev, double* J_host);
+int loop_slices(qq_ctx* c, const Spinor y[2], const Spinor b[2], int ksub, double* J_host);
 
 namespace {
 
@@ -64,7 +63,6 @@ constexpr int kCombineOut = 16;     // outputs per combine launch
 constexpr double kPairTol = 1e-8;   // eigtol, Q/disconloops.f90:1638
 constexpr double kResTolM = 1e-8;   // eigtoltemp, :1639
 constexpr double kResTolMp = 1e-5;  // :2812
-constexpr int kWsVal = 4096, kWsJ = 4097, kWsRef = 4098;  // context workspace ids
 
 // out = gamma5 in on `nhalf` half fields (FP64, component-major: element q vh + s,
 // q = 3 spin + colour); gamma5 = [[0, -i], [i, 0]] in 2 x 2 spin blocks.
@@ -559,14 +557,8 @@ int modes_of_mprime(qq_ctx* c, qq_eig* E, EigOp& op, Basis& ev, const std::vecto
 // the device.
 int mode_traces(qq_ctx* c, const qq_eig* E, const double* ze, const double* zo, std::vector<double>& T,
                 std::vector<cd>& proj) {
-  const size_t hn = E->half_nel, nv = c->ref_doubles();
-  const int nt = c->g.n[3], V = 2 * c->g.vh, n = E->num;
-  void *val = nullptr, *Jd = nullptr, *ref = nullptr;
-  QQ_CK(ws_get(c, kWsVal, sizeof(double) * 18 * (size_t)V, &val));
-  QQ_CK(ws_get(c, kWsJ, sizeof(double) * 18 * (size_t)nt, &Jd));
-  QQ_CK(ws_get(c, kWsRef, sizeof(double) * 2 * nv, &ref));
-  double* ye = static_cast<double*>(ref);
-  double* yo = ye + nv;
+  const size_t hn = E->half_nel;
+  const int nt = c->g.n[3], n = E->num;
   Tmp zfe(c, P64), zfo(c, P64), g5e(c, P64), g5o(c, P64);
   QQ_TRY(ref_to_field(c, ze, 0, zfe.sp()));
   QQ_TRY(ref_to_field(c, zo, 1, zfo.sp()));
@@ -584,10 +576,8 @@ int mode_traces(qq_ctx* c, const qq_eig* E, const double* ze, const double* zo, 
       re = g5e.sp();
       ro = g5o.sp();
     }
-    QQ_TRY(field_to_ref(c, re, 0, ye));
-    QQ_TRY(field_to_ref(c, ro, 1, yo));
-    QQ_TRY(loop_slices(c, ye, yo, ze, zo, 0, static_cast<double*>(val), static_cast<double*>(Jd),
-                       T.data() + (size_t)j * 18 * nt));
+    const Spinor y[2] = {re, ro}, z[2] = {zfe.sp(), zfo.sp()};
+    QQ_TRY(loop_slices(c, y, z, 0, T.data() + (size_t)j * 18 * nt));
   }
   return QQ_OK;
 }
@@ -677,20 +667,14 @@ int load_full(qq_ctx* c, const double* e, const double* o, void* full, size_t hn
 }
 
 // ppaverage*: Jtime(2, nt, nsub, 9) at imom = 1 (Fortran order), x and b full vectors in
-// GPU layout, b also in reference layout on the device (be_ref, bo_ref).
-int ppaverage_dev(qq_ctx* c, int p, const double* co, const void* b, const double* be_ref, const double* bo_ref,
-                  const void* x, double kappa, int nsub, double* J) {
-  const size_t hn = (size_t)12 * c->g.vh, nv = c->ref_doubles();
-  const int nt = c->g.n[3], V = 2 * c->g.vh;
+// GPU layout.
+int ppaverage_dev(qq_ctx* c, int p, const double* co, const void* b, const void* x, double kappa, int nsub, double* J) {
+  const size_t hn = (size_t)12 * c->g.vh;
+  const int nt = c->g.n[3];
   Basis P, Y;
   QQ_TRY(krylov_powers(c, b, kappa, hn, poly_powers(p), P));
   QQ_TRY(Y.init(2 * hn, 2));  // sub and y
   QQ_CK(cudaMemsetAsync(Y.v(0), 0, 2 * hn * 16, c->st));
-  void *val = nullptr, *Jd = nullptr, *ref = nullptr;
-  QQ_CK(ws_get(c, kWsVal, sizeof(double) * 18 * (size_t)V, &val));
-  QQ_CK(ws_get(c, kWsJ, sizeof(double) * 18 * (size_t)nt, &Jd));
-  QQ_CK(ws_get(c, kWsRef, sizeof(double) * 2 * nv, &ref));
-  double* ye = static_cast<double*>(ref);
   std::vector<double> T((size_t)18 * nt);
   std::memset(J, 0, sizeof(double) * 2 * (size_t)nt * nsub * 9);
   for (int isub = 1; isub <= nsub; ++isub) {
@@ -698,10 +682,9 @@ int ppaverage_dev(qq_ctx* c, int p, const double* co, const void* b, const doubl
     for (int h = 0; h < 2; ++h)
       QQ_TRY(lin(c, half_of(Y.v(1), hn, h), cimm(1.0), half_of(const_cast<void*>(x), hn, h), cimm(-1.0),
                  half_of(Y.v(0), hn, h)));
-    QQ_TRY(field_to_ref(c, half_of(Y.v(1), hn, 0), 0, ye));
-    QQ_TRY(field_to_ref(c, half_of(Y.v(1), hn, 1), 1, ye + nv));
-    QQ_TRY(loop_slices(c, ye, ye + nv, be_ref, bo_ref, isub == 1 ? 0 : 1, static_cast<double*>(val),
-                       static_cast<double*>(Jd), T.data()));
+    const Spinor y[2] = {half_of(Y.v(1), hn, 0), half_of(Y.v(1), hn, 1)};
+    const Spinor z[2] = {half_of(const_cast<void*>(b), hn, 0), half_of(const_cast<void*>(b), hn, 1)};
+    QQ_TRY(loop_slices(c, y, z, isub == 1 ? 0 : 1, T.data()));
     for (int iop = 0; iop < 9; ++iop)
       for (int it = 0; it < nt; ++it)
         for (int ri = 0; ri < 2; ++ri)
@@ -964,18 +947,15 @@ extern "C" int qq_ppaverage(qq_ctx* c, int p, const double* co, const double* be
   if (nsub < 1 || nsub > 6) return set_error(QQ_BAD_ARG, "nsub must be 1..6");
   if (!c->have_gauge) return set_error(QQ_BAD_ARG, "no gauge field uploaded");
   QQ_CK(cudaSetDevice(c->device));
-  const size_t hn = (size_t)12 * c->g.vh, nv = c->ref_doubles();
-  DevBuf bx, bref;
+  const size_t hn = (size_t)12 * c->g.vh;
+  DevBuf bx;
   QQ_CK(bx.alloc(2 * 2 * hn * 16));
-  QQ_CK(bref.alloc(sizeof(double) * 2 * nv));
   void* b = bx.p;
   void* x = static_cast<char*>(bx.p) + 2 * hn * 16;
   QQ_TRY(load_full(c, be, bo, b, hn));
-  QQ_CK(cudaMemcpyAsync(bref.p, be, sizeof(double) * nv, cudaMemcpyDefault, c->st));
-  QQ_CK(cudaMemcpyAsync(bref.as<double>() + nv, bo, sizeof(double) * nv, cudaMemcpyDefault, c->st));
   QQ_TRY(load_full(c, xe, xo, x, hn));
   std::vector<double> J(2 * (size_t)c->g.n[3] * nsub * 9);
-  QQ_TRY(ppaverage_dev(c, p, co, b, bref.as<double>(), bref.as<double>() + nv, x, kappa, nsub, J.data()));
+  QQ_TRY(ppaverage_dev(c, p, co, b, x, kappa, nsub, J.data()));
   QQ_CK(cudaMemcpy(Jtime, J.data(), sizeof(double) * J.size(), cudaMemcpyDefault));
   return QQ_OK;
 }
@@ -1019,11 +999,11 @@ extern "C" int qq_generalaverage(qq_ctx* c, const qq_eig* m, const qq_eig* mp, c
   // NS: loop operators of the solution, operators 1..4 times kappa
   std::vector<double> NS((size_t)18 * nt);
   {
-    void *val = nullptr, *Jd = nullptr;
-    QQ_CK(ws_get(c, kWsVal, sizeof(double) * 18 * (size_t)2 * c->g.vh, &val));
-    QQ_CK(ws_get(c, kWsJ, sizeof(double) * 18 * (size_t)nt, &Jd));
-    QQ_TRY(loop_slices(c, zref + 2 * nv, zref + 3 * nv, zref, zref + nv, 0, static_cast<double*>(val),
-                       static_cast<double*>(Jd), NS.data()));
+    Tmp x0(c, P64), x1(c, P64);
+    QQ_TRY(ref_to_field(c, zref + 2 * nv, 0, x0.sp()));
+    QQ_TRY(ref_to_field(c, zref + 3 * nv, 1, x1.sp()));
+    const Spinor y[2] = {x0.sp(), x1.sp()}, z[2] = {half_of(zx.p, hn, 0), half_of(zx.p, hn, 1)};
+    QQ_TRY(loop_slices(c, y, z, 0, NS.data()));
     for (int iop = 0; iop < 4; ++iop)
       for (int k = 0; k < 2 * nt; ++k) NS[(size_t)iop * 2 * nt + k] *= kappa;
   }
@@ -1036,9 +1016,9 @@ extern "C" int qq_generalaverage(qq_ctx* c, const qq_eig* m, const qq_eig* mp, c
     QQ_TRY(qq_average(c, zref, zref + nv, zref0.as<double>(), zref0.as<double>(), kappa, nsub, 1, 9, nullptr,
                       PS.data()));
   }
-  QQ_TRY(ppaverage_dev(c, 11, co11, zx.p, zref, zref + nv, zero.p, kappa, nsub, PP.data()));
-  QQ_TRY(ppaverage_dev(c, 5, co5, zx.p, zref, zref + nv, zero.p, kappa, nsub, PP4.data()));
-  QQ_TRY(ppaverage_dev(c, 8, co8, zx.p, zref, zref + nv, zero.p, kappa, nsub, PP7.data()));
+  QQ_TRY(ppaverage_dev(c, 11, co11, zx.p, zero.p, kappa, nsub, PP.data()));
+  QQ_TRY(ppaverage_dev(c, 5, co5, zx.p, zero.p, kappa, nsub, PP4.data()));
+  QQ_TRY(ppaverage_dev(c, 8, co8, zx.p, zero.p, kappa, nsub, PP7.data()));
   for (size_t i = 0; i < PS.size(); ++i) {
     PS[i] = -PS[i];
     PP[i] = -PP[i];
