@@ -179,9 +179,13 @@ __device__ inline void hop(const HopArgs& a, int s, int r, const int* x, cplx<R>
   else
     LIO::load(a.gauge, a.g.vh, 1 - a.pout, MU, sy, u);
   cplx<R> psi[12];
-  SIO::load(a.in_base(r), a.in_nrm(r), a.vh_of(), a.idx_of(sy, r), psi);
+  // the time direction's projectors keep two spins: (1 - gamma_4) the last, (1 + gamma_4)
+  // the first, and only those are read
+  constexpr bool kHalf = MU == 3 && (SP == P64 || SP == P32);
+  if (!kHalf) SIO::load(a.in_base(r), a.in_nrm(r), a.vh_of(), a.idx_of(sy, r), psi);
   cplx<R> h[6], w[6];
   if (cm != (R)0) {
+    if constexpr (kHalf) load_half<SP, 1>(a.in_base(r), a.vh_of(), a.idx_of(sy, r), psi);
     project<MU, -1>(psi, cm, h);
     if (FWD) {
       matvec(u, h, w);
@@ -193,6 +197,7 @@ __device__ inline void hop(const HopArgs& a, int s, int r, const int* x, cplx<R>
     reconstruct_acc<MU, -1>(acc, w);
   }
   if (cp != (R)0) {
+    if constexpr (kHalf) load_half<SP, 0>(a.in_base(r), a.vh_of(), a.idx_of(sy, r), psi);
     project<MU, +1>(psi, cp, h);
     if (FWD) {
       matvec(u, h, w);
@@ -347,8 +352,12 @@ __global__ void __launch_bounds__(128) hop_mrhs_kernel(HopArgs a) {
 // Thread layout: threadIdx.x = (site-in-block) * nrhs + rhs, threadIdx.y = direction
 // group (TPS groups; group t applies the directions mu with mu % TPS == t).  With
 // TPS > 1 the partial sums meet in shared memory and group 0 runs the epilogue.
-template <int SP, int LP, int RECON, int TPS, int EPI>
-__global__ void __launch_bounds__(128) hop_kernel(HopArgs a) {
+// MINB: resident blocks per SM the registers are capped for (1: none).  Uncapped, the FP64
+// kernel takes 226 registers (8 warps per SM, loads of the next hop hoisted); three blocks
+// win where the lattice has many waves of blocks (24^3x48: 92 us against 107), the
+// uncapped one below (16^3x32: 30.8 against 32.8), so the autotuner decides.
+template <int SP, int LP, int RECON, int TPS, int EPI, int MINB>
+__global__ void __launch_bounds__(128, MINB) hop_kernel(HopArgs a) {
   using SIO = SpinorIO<SP>;
   using R = typename SIO::R;
   static_assert(sizeof(typename LinkIO<LP, RECON>::R) == sizeof(R), "link/spinor precision");

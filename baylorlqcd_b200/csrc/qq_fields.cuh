@@ -66,6 +66,29 @@ struct SpinorIO<P32> {
   }
 };
 
+// Spins (0, 1) (HI = 0) or (2, 3) (HI = 1) of a site, components 6 HI .. 6 HI + 5 of v.
+template <int P, int HI>
+__device__ inline void load_half(const void* base, int vh, int s, cplx<typename SpinorIO<P>::R>* v) {
+  static_assert(P == P64 || P == P32, "formats whose planes keep the halves apart");
+  if constexpr (P == P64) {
+    const double2* f = static_cast<const double2*>(base);
+#pragma unroll
+    for (int c = 6 * HI; c < 6 * HI + 6; ++c) {
+      const double2 t = __ldg(f + (size_t)c * vh + s);
+      v[c] = {t.x, t.y};
+    }
+  } else {
+    const float4* f = static_cast<const float4*>(base);
+#pragma unroll
+    for (int q = 3 * HI; q < 3 * HI + 3; ++q) {
+      const float4 t = __ldg(f + (size_t)q * vh + s);
+      const int a = p32_first(q);
+      v[a] = {t.x, t.z};
+      v[a + 3] = {t.y, t.w};
+    }
+  }
+}
+
 // FP16 storage with one FP32 scale per site (max |component|), FP32 arithmetic.
 template <>
 struct SpinorIO<P16> {

@@ -54,15 +54,15 @@ static HopArgs hop_prepare(const HopArgs& a, int per_block, int threads_per_site
   return b;
 }
 
-template <int SP, int LP, int RECON, int TPS>
+template <int SP, int LP, int RECON, int TPS, int MINB = 1>
 static cudaError_t hop_epi(const HopArgs& a, int epi, cudaStream_t st) {
   dim3 blk, grd;
   hop_block_shape(TPS, a.nrhs, a.g.vh, &blk, &grd);
   const HopArgs b = hop_prepare(a, hop_sites_per_block(TPS, a.nrhs), a.nrhs);
   switch (epi) {
-    case EPI_STORE: hop_kernel<SP, LP, RECON, TPS, EPI_STORE><<<grd, blk, 0, st>>>(b); break;
-    case EPI_TWIST: hop_kernel<SP, LP, RECON, TPS, EPI_TWIST><<<grd, blk, 0, st>>>(b); break;
-    case EPI_DBLE: hop_kernel<SP, LP, RECON, TPS, EPI_DBLE><<<grd, blk, 0, st>>>(b); break;
+    case EPI_STORE: hop_kernel<SP, LP, RECON, TPS, EPI_STORE, MINB><<<grd, blk, 0, st>>>(b); break;
+    case EPI_TWIST: hop_kernel<SP, LP, RECON, TPS, EPI_TWIST, MINB><<<grd, blk, 0, st>>>(b); break;
+    case EPI_DBLE: hop_kernel<SP, LP, RECON, TPS, EPI_DBLE, MINB><<<grd, blk, 0, st>>>(b); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
@@ -86,6 +86,11 @@ static cudaError_t hop_tps(const HopArgs& a, int epi, int tps, cudaStream_t st) 
     case 1: return hop_epi<SP, LP, RECON, 1>(a, epi, st);
     case 2: return hop_epi<SP, LP, RECON, 2>(a, epi, st);
     case 4: return hop_epi<SP, LP, RECON, 4>(a, epi, st);
+    case 5:
+    case 6:
+      if constexpr (SP == P64)
+        return tps == 5 ? hop_epi<SP, LP, RECON, 1, 3>(a, epi, st) : hop_epi<SP, LP, RECON, 1, 4>(a, epi, st);
+      return cudaErrorInvalidValue;
     case 32:
     case 64:
     case 96:
@@ -241,6 +246,7 @@ cudaError_t launch_hop(const HopArgs& a, int sp, int recon, int epi, int tps, cu
       case 5: return a.blk ? hop_f2s(a, epi, st) : cudaErrorInvalidValue;  // + staged links
       case 6: return hop_f2a<2, 1>(a, epi, st);  // copy ring, 2 / 3 / 4 stages in flight
       case 7: return hop_f2a<3, 1>(a, epi, st);
+// 5, 6 = FP64 spinors, one group, registers capped for 3 / 4 resident blocks;
       case 8: return hop_f2a<4, 1>(a, epi, st);
       case 9: return hop_f2a<2, 1, 5>(a, epi, st);
       case 10: return hop_f2a<2, 1, 6>(a, epi, st);
@@ -257,7 +263,7 @@ cudaError_t launch_hop(const HopArgs& a, int sp, int recon, int epi, int tps, cu
     if (sp == PB16) return hop_mrhs<PB16, P32, 12>(a, epi, rpt, st);
     return cudaErrorInvalidValue;
   }
-  const int per = tps <= 4 ? 128 / tps : tps;
+  const int per = tps <= 4 ? 128 / tps : tps <= 6 ? 128 : tps;
   if (a.nrhs > per) return cudaErrorInvalidValue;
   if (sp == P64) {
     if (recon == 18) return hop_tps<P64, P64, 18>(a, epi, tps, st);
@@ -482,22 +488,14 @@ cudaError_t launch_spinor_from_ref(const Geom& g, const RefDims& d, int p, const
 cudaError_t launch_spinor_to_ref(const Geom& g, const RefDims& d, int p, Spinor in, double* ref,
                                  cudaStream_t st) {
   count_launch();
-  dim3 blk(128), grd((g.vh + 127) / 128);
   if (in.prec == P64)
-    spinor_to_ref_kernel<P64><<<grd, blk, 0, st>>>(g, d, p, in, ref);
+    spinor_to_ref<P64>(g, d, p, in, ref, st);
   else if (in.prec == P32)
-    spinor_to_ref_kernel<P32><<<grd, blk, 0, st>>>(g, d, p, in, ref);
+    spinor_to_ref<P32>(g, d, p, in, ref, st);
   else if (in.prec == P16)
-    spinor_to_ref_kernel<P16><<<grd, blk, 0, st>>>(g, d, p, in, ref);
+    spinor_to_ref<P16>(g, d, p, in, ref, st);
   else
-    spinor_to_ref_kernel<PB16><<<grd, blk, 0, st>>>(g, d, p, in, ref);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_ref_zero_halo(const RefDims& d, double* ref, cudaStream_t st) {
-  count_launch();
-  if (d.ntotal == d.nvhalf) return cudaSuccess;
-  ref_zero_halo_kernel<<<148, 256, 0, st>>>(d, ref);
+    spinor_to_ref<PB16>(g, d, p, in, ref, st);
   return cudaGetLastError();
 }
 
@@ -508,6 +506,15 @@ cudaError_t launch_gauge_from_ref(const Geom& g, const RefDims& d, const double*
   if (prec == P64 && recon == 18)
     gauge_from_ref_kernel<P64, 18><<<grd, blk, 0, st>>>(g, d, ref, out);
   else if (prec == P64 && recon == 12)
+template <int P>
+static void spinor_to_ref(const Geom& g, const RefDims& d, int p, Spinor in, double* ref, cudaStream_t st) {
+  dim3 blk(128), grd((g.vh + 127) / 128);
+  if (reinterpret_cast<uintptr_t>(ref) % 16 == 0)
+    spinor_to_ref_kernel<P, true><<<grd, blk, 0, st>>>(g, d, p, in, ref);
+  else
+    spinor_to_ref_kernel<P, false><<<grd, blk, 0, st>>>(g, d, p, in, ref);
+}
+
     gauge_from_ref_kernel<P64, 12><<<grd, blk, 0, st>>>(g, d, ref, out);
   else if (prec == P32 && recon == 12)
     gauge_from_ref_kernel<P32, 12><<<grd, blk, 0, st>>>(g, d, ref, out);

@@ -50,7 +50,6 @@ cudaError_t launch_spinor_from_ref(const Geom& g, const RefDims& d, int p, const
                                    Spinor out, cudaStream_t st);
 cudaError_t launch_spinor_to_ref(const Geom& g, const RefDims& d, int p, Spinor in, double* ref,
                                  cudaStream_t st);
-cudaError_t launch_ref_zero_halo(const RefDims& d, double* ref, cudaStream_t st);
 cudaError_t launch_gauge_from_ref(const Geom& g, const RefDims& d, const double* ref, void* out,
                                   int prec, int recon, cudaStream_t st);
 cudaError_t launch_su3_defect(const Geom& g, const RefDims& d, const double* ref,

@@ -44,11 +44,32 @@ __global__ void spinor_from_ref_kernel(Geom g, RefDims d, int p, const double* r
   SpinorIO<PO>::store(out.data, out.norm, g.vh, s, v);
 }
 
-// reference half-vector <- GPU spinor (interior sites only).
-template <int PI>
+// reference half-vector <- GPU spinor, and zeros in the halo slots (isite > nvhalf), as
+// Hsingle's `gout = 0.0_KR` leaves them (Q/diracops.f90:590).  VEC: the array is 16-byte
+// aligned, and a complex number is stored at once: the 48-byte rows of a spin are
+// scattered by the blocked layout, so the stores per sector are what the kernel costs
+// (24^3x48: 41 us with 8-byte stores).
+template <int PI, bool VEC>
 __global__ void spinor_to_ref_kernel(Geom g, RefDims d, int p, Spinor in, double* ref) {
   using R = typename SpinorIO<PI>::R;
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  auto put = [&](size_t k, double re, double im) {
+    if (VEC) {
+      *reinterpret_cast<double2*>(ref + k) = make_double2(re, im);
+    } else {
+      ref[k] = re;
+      ref[k + 1] = im;
+    }
+  };
+  const int nb = d.ntotal - d.nvhalf;
+  const int total = nb * 3 * 4 * 2 * 8;
+  for (int t = s; t < total; t += gridDim.x * blockDim.x) {
+    int r = t;
+    const int c = r % 3; r /= 3;
+    const int ib = r % nb; r /= nb;
+    const int id = r % 4; r /= 4;
+    put(ref_gi(d, 2 * c + 1, d.nvhalf + ib + 1, id + 1, r % 2 + 1, r / 2 + 1), 0.0, 0.0);
+  }
   if (s >= g.vh) return;
   int x[4], isite, ieo, ibleo;
   site_coords(g, p, s, x);
@@ -58,27 +79,8 @@ __global__ void spinor_to_ref_kernel(Geom g, RefDims d, int p, Spinor in, double
 #pragma unroll
   for (int id = 1; id <= 4; ++id)
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const size_t k = ref_gi(d, 2 * c + 1, isite, id, ieo, ibleo);
-      ref[k] = (double)v[3 * (id - 1) + c].re;
-      ref[k + 1] = (double)v[3 * (id - 1) + c].im;
-    }
-}
-
-// Zero the halo slots (isite > nvhalf) of a reference half-vector, as Hsingle's
-// `gout = 0.0_KR` leaves them (Q/diracops.f90:590).
-static __global__ void ref_zero_halo_kernel(RefDims d, double* ref) {
-  const int nb = d.ntotal - d.nvhalf;
-  const int total = nb * 6 * 4 * 2 * 8;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-    int r = t;
-    const int a = r % 6; r /= 6;
-    const int ib = r % nb; r /= nb;
-    const int id = r % 4; r /= 4;
-    const int ieo = r % 2; r /= 2;
-    const int ibleo = r;
-    ref[ref_gi(d, a + 1, d.nvhalf + ib + 1, id + 1, ieo + 1, ibleo + 1)] = 0.0;
-  }
+    for (int c = 0; c < 3; ++c)
+      put(ref_gi(d, 2 * c + 1, isite, id, ieo, ibleo), (double)v[3 * (id - 1) + c].re, (double)v[3 * (id - 1) + c].im);
 }
 
 // GPU gauge field <- reference u(18, ntotal, 4, 2, 16).

@@ -91,7 +91,6 @@ int ref_to_field(qq_ctx* c, const double* ref_dev, int parity, Spinor out) {
 }
 
 int field_to_ref(qq_ctx* c, Spinor in, int parity, double* ref_dev) {
-  QQ_CK(launch_ref_zero_halo(c->rd, ref_dev, c->st));
   QQ_CK(launch_spinor_to_ref(c->g, c->rd, parity, in, ref_dev, c->st));
   return QQ_OK;
 }
@@ -192,11 +191,11 @@ int launch_hop_tuned(qq_ctx* c, const HopArgs& a, int prec, int epi) {
   QQ_CK(tune_flush_buffer(&flush, &flush_bytes));
   int best = 1;
   float best_ms = 1e30f;
-  for (int tps : {1, 2, 32, 64, 96, 128, kShapeMrhs + 2, kShapeMrhs + 3, kShapeMrhs + 4, kShapeF2 + 1,
+  for (int tps : {1, 2, 5, 6, 32, 64, 96, 128, kShapeMrhs + 2, kShapeMrhs + 3, kShapeMrhs + 4, kShapeF2 + 1,
                   kShapeF2 + 2, kShapeF2 + 3, kShapeF2 + 4, kShapeF2 + 5, kShapeF2 + 6, kShapeF2 + 7,
                   kShapeF2 + 8, kShapeF2 + 9, kShapeF2 + 10, kShapeF2 + 11}) {
-    const int per = tps <= 4 ? 128 / tps : tps;
-    if (a.nrhs > per) continue;
+    const int per = tps <= 4 ? 128 / tps : tps <= 6 ? 128 : tps;
+    if (a.nrhs > per || ((tps == 5 || tps == 6) && prec != P64)) continue;
     if (tps >= kShapeF2 + 6) {  // copy ring, every variant (its shared memory pays off from 4 RHS up)
       if (prec != P32 || a.nrhs < 4) continue;
     } else if (tps == kShapeF2 + 5) {  // + links staged in shared memory (block fields, nrhs >= 8)
