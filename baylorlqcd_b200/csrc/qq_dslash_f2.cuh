@@ -581,23 +581,9 @@ __device__ inline void f2a_run(const HopArgs& a, const F2aShared& sh, int s, int
   }
 }
 
-// Thread layout: threadIdx.x = (site-in-block) * G + j, G = nrhs / RPT threads per site.
-// MINB: resident blocks per SM the register allocation is capped for (4: none; 5 and 6
-// trade a few spilled registers for 25-50% more resident warps).
-// MB: hop-matrix layout (0: 5 packed entries per hop, 1: 9 pre-broadcast entries).
-template <int EPI, int D, int RPT, int MINB, int MB = 0>
-__global__ void __launch_bounds__(128, MINB) hop_f2a_kernel(HopArgs a) {
-  extern __shared__ float4 f2a_smem[];
-  const int T = blockDim.x, per = a.per_block, tx = threadIdx.x;
-  const int G = a.nrhs / RPT;
-  F2aShared sh;
-  sh.raw = f2a_smem;
-  sh.mat = sh.raw + per * 24;
-  sh.ring = sh.mat + per * f2a_mat_stride(MB);
-  sh.nbr = reinterpret_cast<int*>(sh.ring + D * RPT * 6 * T);
-  sh.sgn = reinterpret_cast<float*>(sh.nbr + per * 8);
-  const int s0 = blockIdx.x * per;
-  // 1. per (site, hop): neighbour index and sign; copy of the link's recon-12 rows
+// 1. Per (site, hop) of the block's sites: neighbour index and sign; copies of the links'
+// recon-12 rows are started.
+__device__ inline void f2a_tables(const HopArgs& a, const F2aShared& sh, int per, int s0, int T, int tx) {
   for (int k = tx; k < per * 8; k += T) {
     const int sl = k >> 3, h = k & 7, mu = h >> 1;
     const int ss = min(s0 + sl, a.g.vh - 1);  // sites past the end: any valid site, never read
@@ -624,19 +610,11 @@ __global__ void __launch_bounds__(128, MINB) hop_f2a_kernel(HopArgs a) {
 #pragma unroll
     for (int q = 0; q < 3; ++q) cp_async16(sh.raw + k * 3 + q, gl + (size_t)q * a.g.vh);
   }
-  cp_async_commit();
-  __syncthreads();  // the neighbour table
-  const int sl = a.div_nrhs.div(tx);
-  const int j = tx - sl * G;
-  const int s = s0 + sl;
-  const bool act = s < a.g.vh;
-  f2a_issue<0, D, EPI, RPT>(a, sh, s, sl, j, G, T, tx, act);
-  if constexpr (D > 1) f2a_issue<1, D, EPI, RPT>(a, sh, s, sl, j, G, T, tx, act);
-  if constexpr (D > 2) f2a_issue<2, D, EPI, RPT>(a, sh, s, sl, j, G, T, tx, act);
-  if constexpr (D > 3) f2a_issue<3, D, EPI, RPT>(a, sh, s, sl, j, G, T, tx, act);
-  cp_async_wait<D>();  // the link rows (the oldest group) have landed ...
-  __syncthreads();     // ... for every thread of the block
-  // 2. hop matrices: M = U (forward) or U^+ (backward), 18 floats (re, im) row-major
+}
+
+// 2. Hop matrices: M = U (forward) or U^+ (backward), 18 floats (re, im) row-major.
+template <int MB>
+__device__ inline void f2a_matrices(const F2aShared& sh, int per, int T, int tx) {
   for (int k = tx; k < per * 8; k += T) {
     Su3<float> u;
 #pragma unroll
@@ -666,6 +644,38 @@ __global__ void __launch_bounds__(128, MINB) hop_f2a_kernel(HopArgs a) {
       for (int e = 0; e < 5; ++e) dst[e] = make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
     }
   }
+}
+
+// Thread layout: threadIdx.x = (site-in-block) * G + j, G = nrhs / RPT threads per site.
+// MINB: resident blocks per SM the register allocation is capped for (4: none; 5 and 6
+// trade a few spilled registers for 25-50% more resident warps).
+// MB: hop-matrix layout (0: 5 packed entries per hop, 1: 9 pre-broadcast entries).
+template <int EPI, int D, int RPT, int MINB, int MB = 0>
+__global__ void __launch_bounds__(128, MINB) hop_f2a_kernel(HopArgs a) {
+  extern __shared__ float4 f2a_smem[];
+  const int T = blockDim.x, per = a.per_block, tx = threadIdx.x;
+  const int G = a.nrhs / RPT;
+  F2aShared sh;
+  sh.raw = f2a_smem;
+  sh.mat = sh.raw + per * 24;
+  sh.ring = sh.mat + per * f2a_mat_stride(MB);
+  sh.nbr = reinterpret_cast<int*>(sh.ring + D * RPT * 6 * T);
+  sh.sgn = reinterpret_cast<float*>(sh.nbr + per * 8);
+  const int s0 = blockIdx.x * per;
+  f2a_tables(a, sh, per, s0, T, tx);
+  cp_async_commit();
+  __syncthreads();  // the neighbour table
+  const int sl = a.div_nrhs.div(tx);
+  const int j = tx - sl * G;
+  const int s = s0 + sl;
+  const bool act = s < a.g.vh;
+  f2a_issue<0, D, EPI, RPT>(a, sh, s, sl, j, G, T, tx, act);
+  if constexpr (D > 1) f2a_issue<1, D, EPI, RPT>(a, sh, s, sl, j, G, T, tx, act);
+  if constexpr (D > 2) f2a_issue<2, D, EPI, RPT>(a, sh, s, sl, j, G, T, tx, act);
+  if constexpr (D > 3) f2a_issue<3, D, EPI, RPT>(a, sh, s, sl, j, G, T, tx, act);
+  cp_async_wait<D>();  // the link rows (the oldest group) have landed ...
+  __syncthreads();     // ... for every thread of the block
+  f2a_matrices<MB>(sh, per, T, tx);
   __syncthreads();
   double dsum[3] = {0.0, 0.0, 0.0};  // this thread's share of the fused dot products
   if (act) {
@@ -735,6 +745,226 @@ __global__ void __launch_bounds__(128, MINB) hop_f2a_kernel(HopArgs a) {
       dst[2] = t2;
     }
   }
+}
+
+// ---------------------------------------------------------------------------
+// The copy ring for 16-bit spinors (FP16 or BF16 with a norm per site, FP32 arithmetic).
+// A stage is 3 16-byte vectors and the site's norm; a thread widens them when it takes the
+// stage, projects component by component, and the norm scales the reconstruction's
+// coefficient, so widening costs 24 conversions a hop and nothing else.  The register
+// kernels it replaces wait for every hop's loads at half the bytes.
+// ---------------------------------------------------------------------------
+template <int SP>
+__device__ inline void widen16(const uint4* slot, int T, cplx<float>* v) {
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    const uint4 t = slot[q * T];
+    const unsigned w[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      float2 f;
+      if constexpr (SP == P16) {
+        __half2 h;
+        __builtin_memcpy(&h, &w[k], 4);
+        f = __half22float2(h);
+      } else {
+        __nv_bfloat162 h;
+        __builtin_memcpy(&h, &w[k], 4);
+        f = __bfloat1622float2(h);
+      }
+      v[4 * q + k] = {f.x, f.y};
+    }
+  }
+}
+
+// Half spinor (h0, h1) of components v: pairs of real and of imaginary parts.
+template <int MU, int S>
+__device__ inline void project_v(const cplx<float>* v, float2* hre, float2* him) {
+  constexpr float s = (float)S;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    if (MU == 0) {
+      hre[c] = make_float2(v[c].re + s * v[9 + c].re, v[3 + c].re + s * v[6 + c].re);
+      him[c] = make_float2(v[c].im + s * v[9 + c].im, v[3 + c].im + s * v[6 + c].im);
+    } else if (MU == 1) {
+      hre[c] = make_float2(v[c].re + s * v[9 + c].im, v[3 + c].re - s * v[6 + c].im);
+      him[c] = make_float2(v[c].im - s * v[9 + c].re, v[3 + c].im + s * v[6 + c].re);
+    } else if (MU == 2) {
+      hre[c] = make_float2(v[c].re + s * v[6 + c].re, v[3 + c].re - s * v[9 + c].re);
+      him[c] = make_float2(v[c].im + s * v[6 + c].im, v[3 + c].im - s * v[9 + c].im);
+    } else {
+      const int o = S < 0 ? 6 : 0;
+      hre[c] = make_float2(v[o + c].re, v[o + 3 + c].re);
+      him[c] = make_float2(v[o + c].im, v[o + 3 + c].im);
+    }
+  }
+}
+
+struct Ring16 {
+  uint4* data;  // [stage][3][thread]
+  float* norm;  // [stage][thread]
+};
+
+inline size_t ring16_smem_bytes(int per_block, int threads, int depth) {
+  return (size_t)per_block * 8 * 8 + (size_t)16 * per_block * (24 + kF2aMatStride) + (size_t)52 * depth * threads;
+}
+
+// Stage H (hops 0-7, 8 = the EPI_DBLE operand) into ring slot H % D; always one group.
+template <int H, int D, int EPI>
+__device__ inline void ring16_issue(const HopArgs& a, const F2aShared& sh, const Ring16& ring, int s, int sl, int r,
+                                    int T, int tx, bool act) {
+  if constexpr (H < 8 || (H == 8 && EPI == EPI_DBLE)) {
+    if (act) {
+      const int site = H < 8 ? sh.nbr[sl * 8 + H] : s, n = a.vh_of(), e = a.idx_of(site, r);
+      const uint4* f = static_cast<const uint4*>(H < 8 ? a.in_base(r) : a.blk ? a.aux[0] : a.aux[r]) + e;
+      const float* nrm = (H < 8 ? a.in_nrm(r) : a.blk ? a.aux_norm[0] : a.aux_norm[r]) + e;
+      uint4* dst = ring.data + (H % D) * 3 * T + tx;
+#pragma unroll
+      for (int q = 0; q < 3; ++q) cp_async16(dst + q * T, f + (size_t)q * n);
+      cp_async4(ring.norm + (H % D) * T + tx, nrm);
+    }
+  }
+  cp_async_commit();
+}
+
+// acc keeps its second spin pair as (3, 2) during the x and y hops, whose reconstruction
+// exchanges the rows.
+template <int H, int D, int EPI, int SP>
+__device__ inline void ring16_run(const HopArgs& a, const F2aShared& sh, const Ring16& ring, int s, int sl, int r,
+                                  int T, int tx, Pair12& acc) {
+  if constexpr (H < 8) {
+    constexpr int MU = H >> 1;
+    constexpr bool FWD = !(H & 1);
+    if constexpr (H == 4) {
+#pragma unroll
+      for (int q = 3; q < 6; ++q) {
+        acc.re[q] = f2swap(acc.re[q]);
+        acc.im[q] = f2swap(acc.im[q]);
+      }
+    }
+    cp_async_wait<D - 1>();
+    const float sgn = sh.sgn[sl * 8 + H];
+    if (sgn != 0.0f) {
+      const float scale = (MU == 3 ? 2.0f : 1.0f) * sgn * ring.norm[(H % D) * T + tx];
+      const float cm = FWD ? a.c.fmf[MU] : a.c.bmf[MU], cp = FWD ? a.c.fpf[MU] : a.c.bpf[MU];
+      LinkPairs m;
+      {
+        const float4* mp = sh.mat + sl * kF2aMatStride + H * 5;
+        float me[20];
+#pragma unroll
+        for (int e = 0; e < 5; ++e) {
+          const float4 t = mp[e];
+          me[4 * e] = t.x;
+          me[4 * e + 1] = t.y;
+          me[4 * e + 2] = t.z;
+          me[4 * e + 3] = t.w;
+        }
+#pragma unroll
+        for (int e = 0; e < 9; ++e) {
+          m.r[e / 3][e % 3] = f2bc(me[2 * e]);
+          m.i[e / 3][e % 3] = f2bc(me[2 * e + 1]);
+        }
+      }
+      cplx<float> v[12];
+      widen16<SP>(ring.data + (H % D) * 3 * T + tx, T, v);
+      float2 hre[3], him[3], wre[3], wim[3];
+      auto add = [&](float k, float ks) {
+        matvec2(m, hre, him, wre, wim);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          if (MU == 3) {
+            const int q = ks < 0.0f ? 3 + c : c;
+            acc.re[q] = f2fma(f2bc(k), wre[c], acc.re[q]);
+            acc.im[q] = f2fma(f2bc(k), wim[c], acc.im[q]);
+            continue;
+          }
+          const float kk = k * ks;
+          acc.re[c] = f2fma(f2bc(k), wre[c], acc.re[c]);
+          acc.im[c] = f2fma(f2bc(k), wim[c], acc.im[c]);
+          if (MU == 0) {
+            acc.re[3 + c] = f2fma(f2bc(kk), wre[c], acc.re[3 + c]);
+            acc.im[3 + c] = f2fma(f2bc(kk), wim[c], acc.im[3 + c]);
+          } else if (MU == 1) {
+            acc.re[3 + c] = f2fma(make_float2(-kk, kk), wim[c], acc.re[3 + c]);
+            acc.im[3 + c] = f2fma(make_float2(kk, -kk), wre[c], acc.im[3 + c]);
+          } else {
+            acc.re[3 + c] = f2fma(make_float2(kk, -kk), wre[c], acc.re[3 + c]);
+            acc.im[3 + c] = f2fma(make_float2(kk, -kk), wim[c], acc.im[3 + c]);
+          }
+        }
+      };
+      if (cm != 0.0f) {
+        project_v<MU, -1>(v, hre, him);
+        add(scale * cm, -1.0f);
+      }
+      if (cp != 0.0f) {
+        project_v<MU, +1>(v, hre, him);
+        add(scale * cp, 1.0f);
+      }
+    }
+    ring16_issue<H + D, D, EPI>(a, sh, ring, s, sl, r, T, tx, true);
+    ring16_run<H + 1, D, EPI, SP>(a, sh, ring, s, sl, r, T, tx, acc);
+  }
+}
+
+// Thread layout: threadIdx.x = (site-in-block) * nrhs + rhs.
+template <int SP, int EPI, int D>
+__global__ void __launch_bounds__(128, 4) hop_ring16_kernel(HopArgs a) {
+  extern __shared__ float4 f2a_smem[];
+  const int T = blockDim.x, per = a.per_block, tx = threadIdx.x;
+  F2aShared sh;
+  sh.raw = f2a_smem;
+  sh.mat = sh.raw + per * 24;
+  Ring16 ring;
+  ring.data = reinterpret_cast<uint4*>(sh.mat + per * kF2aMatStride);
+  ring.norm = reinterpret_cast<float*>(ring.data + D * 3 * T);
+  sh.ring = nullptr;
+  sh.nbr = reinterpret_cast<int*>(ring.norm + D * T);
+  sh.sgn = reinterpret_cast<float*>(sh.nbr + per * 8);
+  const int s0 = blockIdx.x * per;
+  f2a_tables(a, sh, per, s0, T, tx);
+  cp_async_commit();
+  __syncthreads();  // the neighbour table
+  const int sl = a.div_nrhs.div(tx), r = tx - sl * a.nrhs, s = s0 + sl;
+  const bool act = s < a.g.vh;
+  ring16_issue<0, D, EPI>(a, sh, ring, s, sl, r, T, tx, act);
+  ring16_issue<1, D, EPI>(a, sh, ring, s, sl, r, T, tx, act);
+  ring16_issue<2, D, EPI>(a, sh, ring, s, sl, r, T, tx, act);
+  if constexpr (D > 3) ring16_issue<3, D, EPI>(a, sh, ring, s, sl, r, T, tx, act);
+  cp_async_wait<D>();  // the link rows have landed ...
+  __syncthreads();     // ... for every thread of the block
+  f2a_matrices<0>(sh, per, T, tx);
+  __syncthreads();
+  if (!act) return;
+  Pair12 acc;
+#pragma unroll
+  for (int q = 0; q < 6; ++q) acc.re[q] = acc.im[q] = make_float2(0.0f, 0.0f);
+  ring16_run<0, D, EPI, SP>(a, sh, ring, s, sl, r, T, tx, acc);
+  cplx<float> o[12], g[12];
+#pragma unroll
+  for (int q = 0; q < 6; ++q) {
+    const int c = p32_first(q);
+    o[c] = {acc.re[q].x, acc.im[q].x};
+    o[c + 3] = {acc.re[q].y, acc.im[q].y};
+  }
+  if constexpr (EPI == EPI_TWIST) {
+#pragma unroll
+    for (int c = 0; c < 6; ++c) {
+      const cplx<float> u = o[c], l = o[6 + c];
+      o[c] = csub(u, cscale(a.af, l));
+      o[6 + c] = cadd(l, cscale(a.af, u));
+    }
+  } else if constexpr (EPI == EPI_DBLE) {
+    cp_async_wait<D - 1>();  // stage 8
+    widen16<SP>(ring.data + (8 % D) * 3 * T + tx, T, g);
+    const float nrm = ring.norm[(8 % D) * T + tx], f1 = a.f1f * nrm, f2 = a.f2f * nrm;
+#pragma unroll
+    for (int c = 0; c < 6; ++c) {
+      o[c] = csub(cadd(cscale(f1, g[c]), cscale(f2, g[6 + c])), cscale(a.f3f, o[c]));
+      o[6 + c] = csub(csub(cscale(f1, g[6 + c]), cscale(f2, g[c])), cscale(a.f3f, o[6 + c]));
+    }
+  }
+  SpinorIO<SP>::store(a.blk ? a.out[0] : a.out[r], a.blk ? a.out_norm[0] : a.out_norm[r], a.vh_of(), a.idx_of(s, r), o);
 }
 
 // Thread layout as hop_mrhs_kernel: threadIdx.x = (site-in-block) * G + j, G = nrhs / RPT.

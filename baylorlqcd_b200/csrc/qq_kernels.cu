@@ -221,7 +221,32 @@ static cudaError_t hop_f2a(const HopArgs& a, int epi, cudaStream_t st) {
   }
 }
 
+// Copy ring for 16-bit spinors, D stages in flight per thread.
+template <int SP, int EPI, int D>
+static cudaError_t hop_ring16_epi(const HopArgs& b, size_t smem, cudaStream_t st) {
+  const cudaError_t e = smem_attr_once((const void*)hop_ring16_kernel<SP, EPI, D>, 227 * 1024);
+  if (e != cudaSuccess) return e;
+  hop_ring16_kernel<SP, EPI, D>
+      <<<(b.g.vh + b.per_block - 1) / b.per_block, b.per_block * b.nrhs, smem, st>>>(b);
+  return cudaGetLastError();
+}
+
+template <int SP, int D>
+static cudaError_t hop_ring16(const HopArgs& a, int epi, cudaStream_t st) {
+  const int per_block = hop_sites_per_block(1, a.nrhs);
+  const HopArgs b = hop_prepare(a, per_block, a.nrhs);
+  const size_t smem = ring16_smem_bytes(per_block, per_block * a.nrhs, D);
+  if (smem > 227 * 1024) return cudaErrorInvalidValue;
+  switch (epi) {
+    case EPI_STORE: return hop_ring16_epi<SP, EPI_STORE, D>(b, smem, st);
+    case EPI_TWIST: return hop_ring16_epi<SP, EPI_TWIST, D>(b, smem, st);
+    case EPI_DBLE: return hop_ring16_epi<SP, EPI_DBLE, D>(b, smem, st);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
 // tps: 1, 2, 4 = register kernel with that many direction groups per site;
+// 5, 6 = FP64 spinors, one group, registers capped for 3 / 4 resident blocks;
 // 32, 64, 96, 128 = staged kernel with that many threads per block;
 // kShapeMrhs + RPT (RPT = 2, 3, 4) = block fields with RPT right-hand sides per thread
 // (FP32 / FP16 spinors, nrhs divisible by RPT);
@@ -229,11 +254,16 @@ static cudaError_t hop_f2a(const HopArgs& a, int epi, cudaStream_t st) {
 // on block fields only); kShapeF2 + 4 = the same, loads a hop ahead; + 5 = links staged
 // in shared memory (block fields); + 6, 7, 8 = copy ring with 2, 3, 4 stages in flight;
 // + 9, 10 = copy ring with 2 stages, registers capped for 5 / 6 resident blocks;
+// (+ 7 and + 8 on 16-bit spinors too);
 // + 11 = copy ring with 3 stages and pre-broadcast hop matrices read row by row.
 cudaError_t launch_hop(const HopArgs& a, int sp, int recon, int epi, int tps, cudaStream_t st) {
   count_launch();
   const int maxr = a.blk ? kMaxBatch : kMaxRhs;
   if (a.nrhs < 1 || a.nrhs > maxr) return cudaErrorInvalidValue;
+  if (has_norm(sp) && (tps == kShapeF2 + 7 || tps == kShapeF2 + 8)) {  // 16-bit copy ring
+    if (sp == P16) return tps == kShapeF2 + 7 ? hop_ring16<P16, 3>(a, epi, st) : hop_ring16<P16, 4>(a, epi, st);
+    return tps == kShapeF2 + 7 ? hop_ring16<PB16, 3>(a, epi, st) : hop_ring16<PB16, 4>(a, epi, st);
+  }
   if (tps > kShapeF2) {
     const int rpt = tps - kShapeF2;
     if (sp != P32 || ((rpt == 2 || rpt == 3) && (a.nrhs % rpt != 0 || !a.blk)))
@@ -246,7 +276,6 @@ cudaError_t launch_hop(const HopArgs& a, int sp, int recon, int epi, int tps, cu
       case 5: return a.blk ? hop_f2s(a, epi, st) : cudaErrorInvalidValue;  // + staged links
       case 6: return hop_f2a<2, 1>(a, epi, st);  // copy ring, 2 / 3 / 4 stages in flight
       case 7: return hop_f2a<3, 1>(a, epi, st);
-// 5, 6 = FP64 spinors, one group, registers capped for 3 / 4 resident blocks;
       case 8: return hop_f2a<4, 1>(a, epi, st);
       case 9: return hop_f2a<2, 1, 5>(a, epi, st);
       case 10: return hop_f2a<2, 1, 6>(a, epi, st);
@@ -485,6 +514,15 @@ cudaError_t launch_spinor_from_ref(const Geom& g, const RefDims& d, int p, const
   return cudaGetLastError();
 }
 
+template <int P>
+static void spinor_to_ref(const Geom& g, const RefDims& d, int p, Spinor in, double* ref, cudaStream_t st) {
+  dim3 blk(128), grd((g.vh + 127) / 128);
+  if (reinterpret_cast<uintptr_t>(ref) % 16 == 0)
+    spinor_to_ref_kernel<P, true><<<grd, blk, 0, st>>>(g, d, p, in, ref);
+  else
+    spinor_to_ref_kernel<P, false><<<grd, blk, 0, st>>>(g, d, p, in, ref);
+}
+
 cudaError_t launch_spinor_to_ref(const Geom& g, const RefDims& d, int p, Spinor in, double* ref,
                                  cudaStream_t st) {
   count_launch();
@@ -506,15 +544,6 @@ cudaError_t launch_gauge_from_ref(const Geom& g, const RefDims& d, const double*
   if (prec == P64 && recon == 18)
     gauge_from_ref_kernel<P64, 18><<<grd, blk, 0, st>>>(g, d, ref, out);
   else if (prec == P64 && recon == 12)
-template <int P>
-static void spinor_to_ref(const Geom& g, const RefDims& d, int p, Spinor in, double* ref, cudaStream_t st) {
-  dim3 blk(128), grd((g.vh + 127) / 128);
-  if (reinterpret_cast<uintptr_t>(ref) % 16 == 0)
-    spinor_to_ref_kernel<P, true><<<grd, blk, 0, st>>>(g, d, p, in, ref);
-  else
-    spinor_to_ref_kernel<P, false><<<grd, blk, 0, st>>>(g, d, p, in, ref);
-}
-
     gauge_from_ref_kernel<P64, 12><<<grd, blk, 0, st>>>(g, d, ref, out);
   else if (prec == P32 && recon == 12)
     gauge_from_ref_kernel<P32, 12><<<grd, blk, 0, st>>>(g, d, ref, out);

@@ -197,7 +197,8 @@ int launch_hop_tuned(qq_ctx* c, const HopArgs& a, int prec, int epi) {
     const int per = tps <= 4 ? 128 / tps : tps <= 6 ? 128 : tps;
     if (a.nrhs > per || ((tps == 5 || tps == 6) && prec != P64)) continue;
     if (tps >= kShapeF2 + 6) {  // copy ring, every variant (its shared memory pays off from 4 RHS up)
-      if (prec != P32 || a.nrhs < 4) continue;
+      const bool ring16 = has_norm(prec) && (tps == kShapeF2 + 7 || tps == kShapeF2 + 8);
+      if ((prec != P32 && !ring16) || a.nrhs < 4) continue;
     } else if (tps == kShapeF2 + 5) {  // + links staged in shared memory (block fields, nrhs >= 8)
       if (prec != P32 || !a.blk || a.nrhs < 8) continue;
     } else if (tps == kShapeF2 + 4) {  // pipelined packed kernel, one RHS per thread

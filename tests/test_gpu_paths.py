@@ -1,0 +1,114 @@
+"""Edges of the GPU kernels behind the solvers, the network's training and the layout
+conversion: column counts of the one-launch orthonormalisation, blocks of right-hand
+sides that share reliable updates, pairs beyond one group of the network's layers, and
+device arrays that are not 16-byte aligned."""
+import numpy as np
+import pytest
+
+import oracle
+from qqtest import golden_gauge, random_half
+
+pytestmark = pytest.mark.gpu
+
+DIMS, BC = (4, 4, 4, 8), (1, 1, 1, -1)
+KAPPA = (0.130, 0.01)
+
+
+@pytest.fixture(scope="module")
+def pair():
+    import baylorlqcd_b200 as qq
+
+    ol = oracle.OracleLattice(*DIMS, bc=BC)
+    _, u = golden_gauge(DIMS, ol.ntotal, seed=41, eps=0.3)
+    ol.set_gauge(u)
+    lat = qq.Lattice(*DIMS, bc=BC)
+    lat.gauge_upload(u, recon=18)
+    yield ol, lat
+    lat.close()
+
+
+def interior_rel(a, b, nv):
+    return np.linalg.norm((a - b)[..., :nv, :]) / np.linalg.norm(b[..., :nv, :])
+
+
+@pytest.mark.parametrize("m,k", [(2, 1), (9, 3), (17, 6), (66, 20), (127, 40)])
+def test_gmresdr_column_counts(pair, m, k):
+    """Basis sizes on both sides of the kernel's splits: fewer columns than its 16 warps
+    (whose spare warps share the elements), 16 and 17, 64 and 65 (four or eight columns a
+    warp), and the largest.  Both solve to 1e-11, and the operator's condition at this
+    kappa is below 1e2: solutions agree to 1e-8."""
+    ol, lat = pair
+    be, bo = random_half(ol.ntotal, ol.nvhalf, 5), random_half(ol.ntotal, ol.nvhalf, 6)
+    xe, xo, info = lat.fermprop(be, bo, KAPPA, inverter=5, resmax=1e-11, nGMRES=(m, k))
+    we, wo, st, _ = ol.fermprop(be, bo, KAPPA, inverter=5, resmax=1e-11, nGMRES=(30, 10))
+    assert info.status == 0 and st == 0
+    assert interior_rel(xe, we, ol.nvhalf) < 1e-8 and interior_rel(xo, wo, ol.nvhalf) < 1e-8
+
+
+@pytest.mark.parametrize("nrhs,block,precision", [(1, 1, 32), (5, 3, 32), (33, 32, 32), (5, 8, 16), (3, 2, 64)])
+def test_batch_blocks_share_updates(pair, nrhs, block, precision):
+    """Every right-hand side of every block, with the last block short: converged by the
+    batched iteration (16 bits may be finished by FP32) and equal to the oracle's solution
+    to the tolerance times the operator's condition."""
+    ol, lat = pair
+    be = np.stack([random_half(ol.ntotal, ol.nvhalf, 50 + i) for i in range(nrhs)])
+    bo = np.stack([random_half(ol.ntotal, ol.nvhalf, 150 + i) for i in range(nrhs)])
+    xe, xo, infos = lat.fermprop_batch(be, bo, KAPPA, precision=precision, rhs_block=block, tol=1e-10, deflate=0)
+    for i in range(nrhs):
+        assert infos[i].status == 0 and infos[i].true_rel <= 1e-10 and infos[i].finished_by in (0, 32)
+    for i in {0, nrhs - 1}:
+        we, wo, st, _ = ol.fermprop(be[i], bo[i], KAPPA, inverter=5, resmax=1e-12, nGMRES=(30, 10))
+        assert interior_rel(xe[i], we, ol.nvhalf) < 1e-8 and interior_rel(xo[i], wo, ol.nvhalf) < 1e-8
+
+
+@pytest.mark.parametrize("precision,tol", [(16, 2e-3), (-16, 1.5e-2)])
+@pytest.mark.parametrize("nrhs", [1, 5, 12, 24, 32])
+@pytest.mark.parametrize("shape", [307, 308])
+def test_copy_ring_16bit(pair, shape, nrhs, precision, tol):
+    """The 16-bit copy ring against the oracle's FP64 Hsingle, with the tolerances of the
+    other 16-bit shapes (11 and 8 significant bits against a site's norm); 5 right-hand
+    sides leave the last block partly empty.  128 sites of a parity."""
+    ol, lat = pair
+    gin = np.stack([random_half(ol.ntotal, ol.nvhalf, 500 + i) for i in range(nrhs)])
+    for idag, gblclr in ((0, 1), (1, 2)):
+        out = lat.hsingle_block(gin, idag, gblclr, precision=precision, shape=shape)
+        for k in {0, nrhs - 1}:
+            ref = ol.hsingle(gin[k], idag, gblclr)[..., : ol.nvhalf, :]
+            assert np.abs(out[k][..., : ol.nvhalf, :] - ref).max() < tol * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("channels", [(4, 4), (4, 8, 16, 4), (4, 16, 16, 4)])
+def test_gradient_of_more_pairs_than_a_group(pair, channels):
+    """Pairs go through the layers in groups of at most eight.  The loss and the gradient
+    of nine are the means of the single ones: the FP32 fields are the same but for the
+    residual's scale 1/9 (a relative 2^-24 per element), and the sums are FP64."""
+    import baylorlqcd_b200 as qq
+
+    ol, lat = pair
+    net = qq.Net(channels, seed=3)
+    b = np.stack([random_half(ol.ntotal, ol.nvhalf, 300 + i) for i in range(9)])
+    x = np.stack([random_half(ol.ntotal, ol.nvhalf, 400 + i) for i in range(9)])
+    loss, grad = net.loss_grad(lat, b, x)
+    one = [net.loss_grad(lat, b[i:i + 1], x[i:i + 1]) for i in range(9)]
+    net.close()
+    want = np.mean([g for _, g in one], axis=0)
+    assert abs(loss - np.mean([v for v, _ in one])) <= 1e-12 * abs(loss)
+    assert np.abs(grad - want).max() <= 1e-6 * np.abs(want).max()
+
+
+def test_unaligned_device_arrays(pair):
+    """Reference-layout device arrays 8 bytes off a 16-byte boundary, in and out: the same
+    values, halo slots zeroed."""
+    import torch
+
+    ol, lat = pair
+    g = random_half(ol.ntotal, ol.nvhalf, 7)
+    want = lat.hdbletm(g, 0, KAPPA)
+    n = g.size
+    gin = torch.zeros(n + 1, dtype=torch.float64, device="cuda")
+    out = torch.full((n + 1,), 3.0, dtype=torch.float64, device="cuda")
+    gin[1:] = torch.from_numpy(g).cuda().flatten()
+    torch.cuda.synchronize()
+    lat.hdbletm(gin[1:], 0, KAPPA, out=out[1:])
+    assert np.array_equal(out[1:].cpu().numpy().reshape(g.shape), want)
+    assert out[0].item() == 3.0
