@@ -151,6 +151,8 @@ int launch_hop_tuned(qq_ctx* c, const HopArgs& a, int prec, int epi);
 int hop_tune_key(qq_ctx* c, const HopArgs& a, int prec, int epi);
 int op_hsingle(qq_ctx* c, Spinor out, Spinor in, int idag, int pout);
 int op_hsingle_multi(qq_ctx* c, const Spinor* out, const Spinor* in, int n, int idag, int pout);
+// The arguments of Hdbletm's two launches for one right-hand side, without the fields.
+void hop_pair_args(qq_ctx* c, int prec, int idag, const double kappa[2], HopArgs* h1, HopArgs* h2, int* epi);
 // he = Hdbletm(ge), tmp is an odd-parity temporary of the same precision.
 int op_dbletm(qq_ctx* c, Spinor out, Spinor in, Spinor tmp, int idag, const double kappa[2]);
 // out = gamma5mult(in) - sigma in (Q/diracops.f90:1750-1860), tmp odd-parity.

@@ -351,12 +351,11 @@ static __global__ void bicg_scalar_kernel(double* S, const int* slots, const dou
 }
 
 // <rhat, r> of right-hand side k's slot of two block fields, per-block partials (re,
-// im, 0) at partial[block * 3]; skipped unless bit k of *pred (the insert mask) is set.
+// im, 0) at partial[block * 3].
 template <int P>
 __global__ void __launch_bounds__(kRedThreads) slot_dot_kernel(int vh, int nb, int k, Spinor a, Spinor b,
-                                                              const unsigned* pred, double* partial) {
+                                                              double* partial) {
   using IO = SpinorIO<P>;
-  if (pred && !((*pred >> k) & 1u)) return;
   const int n = vh * nb;
   double re = 0.0, im = 0.0;
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < vh; s += gridDim.x * blockDim.x) {
@@ -387,13 +386,28 @@ __global__ void __launch_bounds__(kRedThreads) slot_dot_kernel(int vh, int nb, i
   }
 }
 
-// After right-hand side k's residual was re-inserted (bit k of the insert mask, or
-// unconditionally when `always`): rho' = <rhat, r> from slot_dot_kernel's partials
-// (fixed-order sum), then beta and rho as at ST_BETA -- or, at a restart (rhat was set
-// to the same residual), rho = ||r||^2 and beta = 0.  One block of 256 threads.
-static __global__ void reliable_rho_kernel(double* S, const int* slots, unsigned* ctl, int k,
-                                           const double* partial, int nblocks, int always) {
-  if (!always && !((ctl[CTL_INSERT] >> k) & 1u)) return;
+// rho' = <rhat, r> = (re, im) of right-hand side k's re-inserted residual: beta and rho as
+// at ST_BETA -- or, at a restart (rhat was set to the same residual), rho = ||r||^2 and
+// beta = 0.
+__device__ inline void reliable_rho(double* S, unsigned* ctl, int k, double re, double im) {
+  double* s = S + (size_t)k * kScal;
+  const unsigned bit = 1u << k;
+  if (ctl[CTL_RESTART] & bit) {  // p = r next
+    atomicAnd(&ctl[CTL_RESTART], ~bit);
+    if (!isfinite(re)) return bicg_fail(s, ctl, k, FAIL_NAN);
+    if (!(re > 0.0)) return bicg_fail(s, ctl, k, FAIL_BREAKDOWN);
+    s[SC_RHO] = re;
+    s[SC_RHO + 1] = 0.0;
+    s[SC_BETA] = s[SC_BETA + 1] = 0.0;
+    s[SC_RHATN] = sqrt(re);
+    return;
+  }
+  bicg_beta(s, ctl, k, re, im, sqrt(s[SC_R2]));
+}
+
+// The same from slot_dot_kernel's partials, after the host re-inserted right-hand side
+// k's residual.  One block of 256 threads.
+static __global__ void reliable_rho_kernel(double* S, unsigned* ctl, int k, const double* partial, int nblocks) {
   __shared__ double red[2][256];
   double a0 = 0.0, a1 = 0.0;
   for (int b = threadIdx.x; b < nblocks; b += blockDim.x) {
@@ -410,21 +424,7 @@ static __global__ void reliable_rho_kernel(double* S, const int* slots, unsigned
     }
     __syncthreads();
   }
-  if (threadIdx.x != 0) return;
-  double* s = S + (size_t)slots[k] * kScal;
-  const unsigned bit = 1u << k;
-  if (ctl[CTL_RESTART] & bit) {  // rhat was set to this residual: rho = ||r||^2, p = r next
-    atomicAnd(&ctl[CTL_RESTART], ~bit);
-    const double rho = red[0][0];
-    if (!isfinite(rho)) return bicg_fail(s, ctl, k, FAIL_NAN);
-    if (!(rho > 0.0)) return bicg_fail(s, ctl, k, FAIL_BREAKDOWN);
-    s[SC_RHO] = rho;
-    s[SC_RHO + 1] = 0.0;
-    s[SC_BETA] = s[SC_BETA + 1] = 0.0;
-    s[SC_RHATN] = sqrt(rho);
-    return;
-  }
-  bicg_beta(s, ctl, k, red[0][0], red[1][0], sqrt(s[SC_R2]));
+  if (threadIdx.x == 0) reliable_rho(S, ctl, k, red[0][0], red[1][0]);
 }
 
 // End of right-hand side k's reliable update, after ||b - A x||^2 has landed in
@@ -433,9 +433,9 @@ static __global__ void reliable_rho_kernel(double* S, const int* slots, unsigned
 // residual (rmax = ||r||).  One thread.
 // Every decision is also appended to right-hand side k's history: hist[k * hmax + j] =
 // the j-th true relative residual, hist_its[k * hmax + j] = the iterations done then.
-static __global__ void reliable_decide_kernel(double* S, const int* slots, unsigned* ctl, int k,
-                                              double tol, double* hist, int* hist_its, int hmax) {
-  double* s = S + (size_t)slots[k] * kScal;
+__device__ inline void reliable_decide(double* S, unsigned* ctl, int k, double tol, double* hist, int* hist_its,
+                                       int hmax) {
+  double* s = S + (size_t)k * kScal;
   const double rn = sqrt(s[SC_T2]);
   const double rel = rn / s[SC_BN];
   s[SC_TRUE] = rel;
@@ -469,7 +469,7 @@ static __global__ void reliable_decide_kernel(double* S, const int* slots, unsig
 }
 
 // After the (predicated) re-insertion: k iterates again unless it converged.
-static __global__ void reliable_resume_kernel(unsigned* ctl, int k) {
+__device__ inline void reliable_resume(unsigned* ctl, int k) {
   const unsigned bit = 1u << k;
   if (ctl[CTL_INSERT] & bit) {
     atomicAnd(&ctl[CTL_INSERT], ~bit);
@@ -477,18 +477,9 @@ static __global__ void reliable_resume_kernel(unsigned* ctl, int k) {
   }
 }
 
-// Conditions of the graph-driven loop (CUDA graph conditional nodes).
-struct CondHandles {
-  cudaGraphConditionalHandle h[kMaxBatch];
-};
-
-// IF node k (right-hand side k's reliable update) runs when k is pending.
-static __global__ void reliable_conds_kernel(const unsigned* ctl, CondHandles hs, int nb) {
-  const int k = threadIdx.x;
-  if (k < nb) {
-    const unsigned pend = ctl[CTL_PENDING] & ~ctl[CTL_DONE];
-    cudaGraphSetConditional(hs.h[k], (pend >> k) & 1u);
-  }
+// IF node of the graph-driven loop: a right-hand side is pending.
+static __global__ void reliable_cond_kernel(const unsigned* ctl, cudaGraphConditionalHandle h) {
+  cudaGraphSetConditional(h, (ctl[CTL_PENDING] & ~ctl[CTL_DONE]) != 0u ? 1u : 0u);
 }
 
 // WHILE node: another iteration while a right-hand side of `all` can still move and
@@ -504,12 +495,9 @@ static __global__ void loop_cond_kernel(unsigned* ctl, unsigned all, unsigned ma
 // Slot k of a block field <-> a separate FP64 field.
 //   mode 0: block[k] = x (rounded to the block precision)   mode 1: x += block[k]
 //   mode 2: block[k] = 0
-// When `pred` is given the kernel does nothing unless bit k of *pred is set.
 template <int P>
-__global__ void block_slot_kernel(int vh, int nb, int k, Spinor blockf, Spinor x, int mode,
-                                  const unsigned* pred) {
+__global__ void block_slot_kernel(int vh, int nb, int k, Spinor blockf, Spinor x, int mode) {
   using RB = typename SpinorIO<P>::R;
-  if (pred && !((*pred >> k) & 1u)) return;
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < vh; s += gridDim.x * blockDim.x) {
     const int e = s * nb + k, n = vh * nb;
     cplx<RB> b[12];

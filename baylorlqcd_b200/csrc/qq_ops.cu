@@ -255,26 +255,37 @@ int op_hsingle(qq_ctx* c, Spinor out, Spinor in, int idag, int pout) {
   return op_hsingle_multi(c, &out, &in, 1, idag, pout);
 }
 
+// The two launches of Hdbletm: h1 (odd output, epilogue *epi) and h2 (even output,
+// EPI_DBLE), for one right-hand side, without fields.
+void hop_pair_args(qq_ctx* c, int prec, int idag, const double kappa[2], HopArgs* h1, HopArgs* h2, int* epi) {
+  const bool wilson = kappa[1] < 0.00000001;  // Q/diracops.f90:467
+  const double t = 2.0 * kappa[0] * kappa[1];
+  *h1 = hop_base(c, idag, 1, prec);
+  h1->nrhs = 1;
+  h1->a = t;
+  *epi = wilson ? EPI_STORE : EPI_TWIST;
+  *h2 = hop_base(c, idag, 0, prec);
+  h2->nrhs = 1;
+  h2->f1 = 1.0 / (kappa[0] * kappa[0]);
+  h2->f2 = wilson ? 0.0 : 2.0 * kappa[1] / kappa[0];
+  h2->f3 = wilson ? 1.0 : 1.0 / (1.0 + t * t);
+}
+
 int op_dbletm_multi(qq_ctx* c, const Spinor* out, const Spinor* in, const Spinor* tmp, int n,
                     int idag, const double kappa[2]) {
   if (!c->have_gauge) return set_error(QQ_BAD_ARG, "no gauge field uploaded");
   const int prec = in[0].prec;
-  const bool wilson = kappa[1] < 0.00000001;  // Q/diracops.f90:467
   for (int r0 = 0; r0 < n; r0 += kMaxRhs) {
     const int nb = std::min(kMaxRhs, n - r0);
-    HopArgs a = hop_base(c, idag, 1, prec);
-    a.nrhs = nb;
+    HopArgs a, b;
+    int epi = EPI_STORE;
+    hop_pair_args(c, prec, idag, kappa, &a, &b, &epi);
+    a.nrhs = b.nrhs = nb;
     for (int r = 0; r < nb; ++r) {
       a.in[r] = in[r0 + r].data;
       a.in_norm[r] = in[r0 + r].norm;
       a.out[r] = tmp[r0 + r].data;
       a.out_norm[r] = tmp[r0 + r].norm;
-    }
-    a.a = 2.0 * kappa[0] * kappa[1];
-    QQ_TRY(launch_hop_tuned(c, a, prec, wilson ? EPI_STORE : EPI_TWIST));
-    HopArgs b = hop_base(c, idag, 0, prec);
-    b.nrhs = nb;
-    for (int r = 0; r < nb; ++r) {
       b.in[r] = tmp[r0 + r].data;
       b.in_norm[r] = tmp[r0 + r].norm;
       b.out[r] = out[r0 + r].data;
@@ -282,15 +293,7 @@ int op_dbletm_multi(qq_ctx* c, const Spinor* out, const Spinor* in, const Spinor
       b.aux[r] = in[r0 + r].data;
       b.aux_norm[r] = in[r0 + r].norm;
     }
-    b.f1 = 1.0 / (kappa[0] * kappa[0]);
-    if (wilson) {
-      b.f2 = 0.0;
-      b.f3 = 1.0;
-    } else {
-      const double t = 2.0 * kappa[0] * kappa[1];
-      b.f2 = 2.0 * kappa[1] / kappa[0];
-      b.f3 = 1.0 / (1.0 + t * t);
-    }
+    QQ_TRY(launch_hop_tuned(c, a, prec, epi));
     QQ_TRY(launch_hop_tuned(c, b, prec, EPI_DBLE));
   }
   return QQ_OK;
@@ -325,34 +328,22 @@ int op_dbletm_block_impl(qq_ctx* c, Spinor out, Spinor in, Spinor tmp, int nb, i
   if (!c->have_gauge) return set_error(QQ_BAD_ARG, "no gauge field uploaded");
   if (nb < 1 || nb > 32) return set_error(QQ_BAD_ARG, "block of 1..32 right-hand sides");
   const int prec = in.prec;
-  const bool wilson = kappa[1] < 0.00000001;  // Q/diracops.f90:467
-  HopArgs a = hop_base(c, idag, 1, prec);
-  a.nrhs = nb;
-  a.blk = 1;
+  HopArgs a, b;
+  int epi = EPI_STORE;
+  hop_pair_args(c, prec, idag, kappa, &a, &b, &epi);
+  a.nrhs = b.nrhs = nb;
+  a.blk = b.blk = 1;
   a.in[0] = in.data;
   a.in_norm[0] = in.norm;
   a.out[0] = tmp.data;
   a.out_norm[0] = tmp.norm;
-  a.a = 2.0 * kappa[0] * kappa[1];
-  QQ_TRY(launch_hop_tuned(c, a, prec, wilson ? EPI_STORE : EPI_TWIST));
-  HopArgs b = hop_base(c, idag, 0, prec);
-  b.nrhs = nb;
-  b.blk = 1;
   b.in[0] = tmp.data;
   b.in_norm[0] = tmp.norm;
   b.out[0] = out.data;
   b.out_norm[0] = out.norm;
   b.aux[0] = in.data;
   b.aux_norm[0] = in.norm;
-  b.f1 = 1.0 / (kappa[0] * kappa[0]);
-  if (wilson) {
-    b.f2 = 0.0;
-    b.f3 = 1.0;
-  } else {
-    const double t = 2.0 * kappa[0] * kappa[1];
-    b.f2 = 2.0 * kappa[1] / kappa[0];
-    b.f3 = 1.0 / (1.0 + t * t);
-  }
+  QQ_TRY(launch_hop_tuned(c, a, prec, epi));
   if (dot_mode && prec == P32 && fused_blocks) {
     // the fusion depends on the tuned shape: tune first (that launch's output is
     // recomputed below), so the first call of a solve is fused like every later one
