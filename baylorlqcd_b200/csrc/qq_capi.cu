@@ -60,6 +60,13 @@ int store_half(qq_ctx* c, int slot, Spinor f, int parity, double* ref) {
   return QQ_OK;
 }
 
+// The staged output goes to the caller's array; waits for the stream.
+int finish_out(qq_ctx* c, int slot, double* out, double* dev) {
+  QQ_TRY(stage_out_end(c, slot, out, c->ref_doubles(), dev));
+  QQ_CK(cudaStreamSynchronize(c->st));
+  return QQ_OK;
+}
+
 int check_iflag(int iflag) {
   if (iflag != -1) return set_error(QQ_BAD_ARG, "only iflag = -1 (Wilson / twisted mass) is supported");
   return QQ_OK;
@@ -184,8 +191,16 @@ int qq_hsingle(qq_ctx* c, double* gout, const double* gin, int idag, int gblclr)
   if (gblclr != 1 && gblclr != 2) return set_error(QQ_BAD_ARG, "gblclr must be 1 or 2");
   if (idag != 0 && idag != 1) return set_error(QQ_BAD_ARG, "idag must be 0 or 1");
   if (!gout || !gin) return set_error(QQ_BAD_ARG, "null array");
-  Tmp in(c, P64), out(c, P64);
   const int pout = gblclr - 1;
+  const double* di = nullptr;
+  double* dout = nullptr;
+  QQ_TRY(stage_in(c, 1, gin, c->ref_doubles(), &di));
+  QQ_TRY(stage_out_begin(c, 2, gout, c->ref_doubles(), &dout));
+  if (hop_ref_usable(c, dout, di)) {
+    QQ_TRY(op_hsingle_ref(c, dout, di, idag, pout));
+    return finish_out(c, 2, gout, dout);
+  }
+  Tmp in(c, P64), out(c, P64);
   QQ_TRY(load_half(c, 1, gin, 1 - pout, in.sp()));
   QQ_TRY(op_hsingle(c, out.sp(), in.sp(), idag, pout));
   return store_half(c, 2, out.sp(), pout, gout);
@@ -202,7 +217,16 @@ int qq_hdbletm(qq_ctx* c, double* he, const double* ge, int idag, const double k
   QQ_TRY(check_iflag(iflag));
   if (!he || !ge || !kappa) return set_error(QQ_BAD_ARG, "null argument");
   if (idag != 0 && idag != 1) return set_error(QQ_BAD_ARG, "idag must be 0 or 1");
-  Tmp in(c, P64), out(c, P64), tmp(c, P64);
+  const double* di = nullptr;
+  double* dout = nullptr;
+  QQ_TRY(stage_in(c, 1, ge, c->ref_doubles(), &di));
+  QQ_TRY(stage_out_begin(c, 2, he, c->ref_doubles(), &dout));
+  Tmp tmp(c, P64);
+  if (hop_ref_usable(c, dout, di)) {
+    QQ_TRY(op_dbletm_ref(c, dout, di, tmp.sp(), idag, kappa));
+    return finish_out(c, 2, he, dout);
+  }
+  Tmp in(c, P64), out(c, P64);
   QQ_TRY(load_half(c, 1, ge, 0, in.sp()));
   QQ_TRY(op_dbletm(c, out.sp(), in.sp(), tmp.sp(), idag, kappa));
   return store_half(c, 2, out.sp(), 0, he);

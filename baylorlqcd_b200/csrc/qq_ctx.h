@@ -153,6 +153,12 @@ int op_hsingle(qq_ctx* c, Spinor out, Spinor in, int idag, int pout);
 int op_hsingle_multi(qq_ctx* c, const Spinor* out, const Spinor* in, int n, int idag, int pout);
 // The arguments of Hdbletm's two launches for one right-hand side, without the fields.
 void hop_pair_args(qq_ctx* c, int prec, int idag, const double kappa[2], HopArgs* h1, HopArgs* h2, int* epi);
+// FP64 Hsingle and Hdbletm on reference-layout device arrays (qq_hopref.cu).  Usable when
+// both arrays are 16-byte aligned and do not overlap, and hops are neither profiled nor
+// forced to a shape.
+bool hop_ref_usable(qq_ctx* c, const double* out, const double* in);
+int op_hsingle_ref(qq_ctx* c, double* out, const double* in, int idag, int pout);
+int op_dbletm_ref(qq_ctx* c, double* out, const double* in, Spinor tmp, int idag, const double kappa[2]);
 // he = Hdbletm(ge), tmp is an odd-parity temporary of the same precision.
 int op_dbletm(qq_ctx* c, Spinor out, Spinor in, Spinor tmp, int idag, const double kappa[2]);
 // out = gamma5mult(in) - sigma in (Q/diracops.f90:1750-1860), tmp odd-parity.

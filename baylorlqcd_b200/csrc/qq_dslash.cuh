@@ -145,10 +145,11 @@ __device__ inline void reconstruct_acc(cplx<R>* acc, const cplx<R>* w) {
   }
 }
 
-// One hop (forward or backward in direction MU) of right-hand side r at output site s.
-template <int SP, int LP, int RECON, int MU, bool FWD, class R>
-__device__ inline void hop(const HopArgs& a, int s, int r, const int* x, cplx<R>* acc) {
-  using SIO = SpinorIO<SP>;
+// One hop (forward or backward in direction MU) at output site s.  load(y, sy, half, psi)
+// reads the neighbour's spinor, coordinates y and index sy: all of it (half = -1), or its
+// spins (0, 1) (half = 0) or (2, 3) (half = 1).
+template <int SP, int LP, int RECON, int MU, bool FWD, class R, class Load>
+__device__ inline void hop_from(const HopArgs& a, int s, const int* x, cplx<R>* acc, Load load) {
   using LIO = LinkIO<LP, RECON>;
   int y[4] = {x[0], x[1], x[2], x[3]};
   constexpr bool kF = sizeof(R) == 4;
@@ -182,10 +183,10 @@ __device__ inline void hop(const HopArgs& a, int s, int r, const int* x, cplx<R>
   // the time direction's projectors keep two spins: (1 - gamma_4) the last, (1 + gamma_4)
   // the first, and only those are read
   constexpr bool kHalf = MU == 3 && (SP == P64 || SP == P32);
-  if (!kHalf) SIO::load(a.in_base(r), a.in_nrm(r), a.vh_of(), a.idx_of(sy, r), psi);
+  if (!kHalf) load(y, sy, -1, psi);
   cplx<R> h[6], w[6];
   if (cm != (R)0) {
-    if constexpr (kHalf) load_half<SP, 1>(a.in_base(r), a.vh_of(), a.idx_of(sy, r), psi);
+    if (kHalf) load(y, sy, 1, psi);
     project<MU, -1>(psi, cm, h);
     if (FWD) {
       matvec(u, h, w);
@@ -197,7 +198,7 @@ __device__ inline void hop(const HopArgs& a, int s, int r, const int* x, cplx<R>
     reconstruct_acc<MU, -1>(acc, w);
   }
   if (cp != (R)0) {
-    if constexpr (kHalf) load_half<SP, 0>(a.in_base(r), a.vh_of(), a.idx_of(sy, r), psi);
+    if (kHalf) load(y, sy, 0, psi);
     project<MU, +1>(psi, cp, h);
     if (FWD) {
       matvec(u, h, w);
@@ -210,13 +211,23 @@ __device__ inline void hop(const HopArgs& a, int s, int r, const int* x, cplx<R>
   }
 }
 
-// Epilogue of one (site, right-hand side): combine the accumulated hopping term with
-// the twist / Schur-complement factors and store.
-template <int SP, int EPI, class R>
-__device__ inline void hop_finish(const HopArgs& a, int s, int r, const cplx<R>* acc) {
-  using SIO = SpinorIO<SP>;
+// The same with right-hand side r of the launch's input field.
+template <int SP, int LP, int RECON, int MU, bool FWD, class R>
+__device__ inline void hop(const HopArgs& a, int s, int r, const int* x, cplx<R>* acc) {
+  hop_from<SP, LP, RECON, MU, FWD>(a, s, x, acc, [&](const int*, int sy, int half, cplx<R>* psi) {
+    if constexpr (SP == P64 || SP == P32) {
+      if (half == 0) return load_half<SP, 0>(a.in_base(r), a.vh_of(), a.idx_of(sy, r), psi);
+      if (half == 1) return load_half<SP, 1>(a.in_base(r), a.vh_of(), a.idx_of(sy, r), psi);
+    }
+    SpinorIO<SP>::load(a.in_base(r), a.in_nrm(r), a.vh_of(), a.idx_of(sy, r), psi);
+  });
+}
+
+// The epilogue's arithmetic: o from the accumulated hopping term and, for EPI_DBLE, the
+// operand gg.
+template <int EPI, class R>
+__device__ inline void hop_combine(const HopArgs& a, const cplx<R>* acc, const cplx<R>* gg, cplx<R>* o) {
   constexpr bool kF = sizeof(R) == 4;
-  cplx<R> o[12];
   if (EPI == EPI_STORE) {
 #pragma unroll
     for (int c = 0; c < 12; ++c) o[c] = acc[c];
@@ -230,9 +241,6 @@ __device__ inline void hop_finish(const HopArgs& a, int s, int r, const cplx<R>*
       o[9 + c] = cadd(acc[9 + c], cscale(t, acc[3 + c]));
     }
   } else {
-    cplx<R> gg[12];
-    SIO::load(a.blk ? a.aux[0] : a.aux[r], a.blk ? a.aux_norm[0] : a.aux_norm[r], a.vh_of(),
-              a.idx_of(s, r), gg);
     const R f1 = kF ? (R)a.f1f : (R)a.f1, f2 = kF ? (R)a.f2f : (R)a.f2, f3 = kF ? (R)a.f3f : (R)a.f3;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -242,6 +250,17 @@ __device__ inline void hop_finish(const HopArgs& a, int s, int r, const cplx<R>*
       o[9 + c] = csub(csub(cscale(f1, gg[9 + c]), cscale(f2, gg[3 + c])), cscale(f3, acc[9 + c]));
     }
   }
+}
+
+// Epilogue of one (site, right-hand side): combine the accumulated hopping term with
+// the twist / Schur-complement factors and store.
+template <int SP, int EPI, class R>
+__device__ inline void hop_finish(const HopArgs& a, int s, int r, const cplx<R>* acc) {
+  using SIO = SpinorIO<SP>;
+  cplx<R> o[12], gg[12];
+  if (EPI == EPI_DBLE)
+    SIO::load(a.blk ? a.aux[0] : a.aux[r], a.blk ? a.aux_norm[0] : a.aux_norm[r], a.vh_of(), a.idx_of(s, r), gg);
+  hop_combine<EPI>(a, acc, gg, o);
   SIO::store(a.blk ? a.out[0] : a.out[r], a.blk ? a.out_norm[0] : a.out_norm[r], a.vh_of(),
              a.idx_of(s, r), o);
 }

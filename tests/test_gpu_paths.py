@@ -96,9 +96,42 @@ def test_gradient_of_more_pairs_than_a_group(pair, channels):
     assert np.abs(grad - want).max() <= 1e-6 * np.abs(want).max()
 
 
+@pytest.mark.parametrize("dims,bc,recon", [((4, 4, 4, 8), (1, 1, 1, -1), 12), ((4, 4, 4, 8), (0, -1, 1, 0), 18),
+                                           ((8, 8, 8, 12), (1, -1, 1, -1), 18), ((16, 8, 16, 40), (1, 1, 1, -1), 12)])
+def test_operator_on_reference_arrays(dims, bc, recon):
+    """Hsingle and Hdbletm read and write the reference layout directly: each number of
+    threads per site its rule picks below the largest lattices (1024, 3072 and 40,960 sites
+    of a parity), both link storages, fixed and antiperiodic boundaries; FP64 against the
+    oracle at its other tests' 1e-13."""
+    import baylorlqcd_b200 as qq
+
+    ol = oracle.OracleLattice(*dims, bc=bc)
+    _, u = golden_gauge(dims, ol.ntotal, seed=43, eps=0.6)
+    ol.set_gauge(u)
+    lat = qq.Lattice(*dims, bc=bc)
+    lat.gauge_upload(u, recon=recon)
+    g = random_half(ol.ntotal, ol.nvhalf, 8)
+    for idag, gblclr in ((0, 1), (1, 2)):
+        want = ol.hsingle(g, idag, gblclr)[..., : ol.nvhalf, :]
+        got = lat.hsingle(g, idag, gblclr)
+        assert np.abs(got[..., : ol.nvhalf, :] - want).max() <= 1e-13 * np.abs(want).max()
+        assert not got[..., ol.nvhalf:, :].any()
+    for kappa in ((0.15, 0.0), (0.15, 0.02)):
+        want = ol.hdbletm(g, 0, kappa)[..., : ol.nvhalf, :]
+        got = lat.hdbletm(g, 0, kappa)[..., : ol.nvhalf, :]
+        assert np.abs(got - want).max() <= 1e-13 * np.abs(want).max()
+    same = g.copy()  # in place: through the GPU layout
+    lat.hdbletm(same, 0, kappa, out=same)
+    assert np.abs(same[..., : ol.nvhalf, :] - want).max() <= 1e-13 * np.abs(want).max()
+    lat.close()
+
+
 def test_unaligned_device_arrays(pair):
-    """Reference-layout device arrays 8 bytes off a 16-byte boundary, in and out: the same
-    values, halo slots zeroed."""
+    """Reference-layout device arrays 8 bytes off a 16-byte boundary, in and out, take the
+    path through the GPU layout; aligned ones are read and written directly.  The same
+    values but for the order of the 24 products a component sums in each of the two hops:
+    2 * 24 * 2^-53 of the sum of their magnitudes, itself below 20 times the largest
+    component, is 1e-13 of that.  Halo slots are zeroed on both."""
     import torch
 
     ol, lat = pair
@@ -110,5 +143,7 @@ def test_unaligned_device_arrays(pair):
     gin[1:] = torch.from_numpy(g).cuda().flatten()
     torch.cuda.synchronize()
     lat.hdbletm(gin[1:], 0, KAPPA, out=out[1:])
-    assert np.array_equal(out[1:].cpu().numpy().reshape(g.shape), want)
+    got = out[1:].cpu().numpy().reshape(g.shape)
+    assert np.abs(got - want).max() <= 1e-13 * np.abs(want).max()
+    assert not got[..., ol.nvhalf:, :].any() and not want[..., ol.nvhalf:, :].any()
     assert out[0].item() == 3.0
