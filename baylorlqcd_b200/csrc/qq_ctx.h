@@ -205,6 +205,11 @@ struct SolveStats {
   std::vector<std::complex<double>> ritz;
 };
 
+// w <- normalised (I - V V^H) w against the first nv <= 127 vectors of V (twice); hcol
+// (device, 2 (nv + 1) doubles, or null) receives V^H w and the norm (qq_arnoldi.cu).
+constexpr int kOrthScratch = 513;  // doubles of ws, zeroed before its first use
+int op_orthonormalize(qq_ctx* c, int pb, const BasisArgs& V, int nv, void* w, double* hcol, double* ws);
+
 // Reference-faithful FP64 GMRES-DR (Q/inverters.f90:2871-3572 semantics).
 int gmresdr_fp64(qq_ctx* c, Spinor phi, Spinor x, int m, int k, double resmax, int itermin,
                  const double kappa[2], DeflSpace* defl, SolveStats* st);

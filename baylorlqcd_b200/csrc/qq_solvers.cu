@@ -30,85 +30,62 @@ struct Arnoldi {
   int pb;
   int m;         // Krylov dimension (m+1 vectors)
   size_t nel;    // 16-byte elements per vector
-  DevBuf V, H, hscr, y;
-  DevBuf Pdev;  // restart rotation ((m+1) x (k+1), k < m), allocated once
+  DevBuf V, small;
+  double* H = nullptr;     // (m+1) x m, column-major
+  double* y = nullptr;     // least-squares solution
+  double* Pdev = nullptr;  // restart rotation ((m+1) x (k+1), k < m)
+  double* orth = nullptr;  // op_orthonormalize's scratch
   // Krylov operator: Hdbletm, or gamma5mult - g5shift (gmresdrshift)
   bool g5 = false;
   double g5shift = 0.0;
+  size_t h_doubles() const { return 2 * (size_t)(m + 1) * m; }
   int init(qq_ctx* c_, int pb_, int m_) {
     c = c_;
     pb = pb_;
     m = m_;
     nel = (pb == P64 ? (size_t)12 : (size_t)6) * c->g.vh;
     QQ_CK(V.alloc((size_t)(m + 1) * nel * 16));
-    QQ_CK(H.alloc(sizeof(double) * 2 * (size_t)(m + 1) * m));
-    QQ_CK(hscr.alloc(sizeof(double) * 2 * 128));
-    QQ_CK(y.alloc(sizeof(double) * 2 * 256));
-    QQ_CK(Pdev.alloc(sizeof(double) * 2 * (size_t)(m + 1) * m));
+    QQ_CK(small.alloc(sizeof(double) * (2 * h_doubles() + 512 + kOrthScratch)));
+    H = small.as<double>();
+    Pdev = H + h_doubles();
+    y = Pdev + h_doubles();
+    orth = y + 512;
+    QQ_CK(cudaMemsetAsync(orth, 0, sizeof(double) * kOrthScratch, c->st));
     return QQ_OK;
   }
   void* vec(int i) const { return static_cast<char*>(V.p) + (size_t)i * nel * 16; }
   Spinor sp(int i) const { return Spinor{vec(i), nullptr, pb}; }
   BasisArgs basis() const { return BasisArgs{V.p, nel, nel}; }
-  double* col(int j) const { return H.as<double>() + 2 * (size_t)(m + 1) * j; }
+  double* col(int j) const { return H + 2 * (size_t)(m + 1) * j; }
   int zeroH() {
-    QQ_CK(cudaMemsetAsync(H.p, 0, H.bytes, c->st));
+    QQ_CK(cudaMemsetAsync(H, 0, sizeof(double) * h_doubles(), c->st));
     return QQ_OK;
   }
 };
 
 // One Arnoldi step: v_{j+1} = normalised (I - V V^H) A src, H(:, j) filled; src = v_j
 // for GMRES, the preconditioned z_j = M v_j for flexible GMRES.
-int arnoldi_step_from(Arnoldi& A, int j, Spinor src, Spinor tmp_odd, const double kappa[2], double* nrm2_slot) {
+int arnoldi_step_from(Arnoldi& A, int j, Spinor src, Spinor tmp_odd, const double kappa[2]) {
   qq_ctx* c = A.c;
   if (A.g5)
     QQ_TRY(op_g5mult(c, A.sp(j + 1), src, tmp_odd, 0, kappa, A.g5shift));
   else
     QQ_TRY(op_dbletm(c, A.sp(j + 1), src, tmp_odd, 0, kappa));
-  double* part = c->partial.as<double>();
-  const int nv = j + 1;
-  int ng = 0;
-  BasisArgs B = A.basis();
-  double* hcol = A.col(j);
-  double* hscr = A.hscr.as<double>();
-  void* w = A.vec(j + 1);
-  QQ_CK(launch_multidot(A.pb, B, nv, w, part, &ng, c->st));
-  QQ_CK(launch_finalize(part, kRedBlocks, ng * 16, 2 * nv, hcol, 0, c->st));
-  QQ_CK(launch_multiaxpy(A.pb, B, nv, hcol, 1.0, w, w, part, c->st));
-  QQ_CK(launch_multidot(A.pb, B, nv, w, part, &ng, c->st));
-  QQ_CK(launch_finalize(part, kRedBlocks, ng * 16, 2 * nv, hscr, 0, c->st));
-  QQ_CK(launch_multiaxpy(A.pb, B, nv, hscr, 1.0, w, w, part, c->st));
-  QQ_CK(launch_finalize(part, kRedBlocks, 3, 1, nrm2_slot, 0, c->st));
-  QQ_CK(launch_hcol_update(A.H.as<double>(), A.m + 1, j, hscr, nv, nrm2_slot, c->st));
-  QQ_CK(launch_normalize(A.pb, A.nel, w, w, nrm2_slot, c->st));
-  return QQ_OK;
+  return op_orthonormalize(c, A.pb, A.basis(), j + 1, A.vec(j + 1), A.col(j), A.orth);
 }
 
-int arnoldi_step(Arnoldi& A, int j, Spinor tmp_odd, const double kappa[2], double* nrm2_slot) {
-  return arnoldi_step_from(A, j, A.sp(j), tmp_odd, kappa, nrm2_slot);
+int arnoldi_step(Arnoldi& A, int j, Spinor tmp_odd, const double kappa[2]) {
+  return arnoldi_step_from(A, j, A.sp(j), tmp_odd, kappa);
 }
 
 // Re-orthogonalise vector `idx` of the basis against vectors [0, idx) and normalise.
-int reorth(Arnoldi& A, int idx, double* nrm2_slot) {
-  qq_ctx* c = A.c;
-  double* part = c->partial.as<double>();
-  double* hscr = A.hscr.as<double>();
-  BasisArgs B = A.basis();
-  void* w = A.vec(idx);
-  int ng = 0;
-  for (int pass = 0; pass < 2; ++pass) {
-    QQ_CK(launch_multidot(A.pb, B, idx, w, part, &ng, c->st));
-    QQ_CK(launch_finalize(part, kRedBlocks, ng * 16, 2 * idx, hscr, 0, c->st));
-    QQ_CK(launch_multiaxpy(A.pb, B, idx, hscr, 1.0, w, w, part, c->st));
-  }
-  QQ_CK(launch_finalize(part, kRedBlocks, 3, 1, nrm2_slot, 0, c->st));
-  QQ_CK(launch_normalize(A.pb, A.nel, w, w, nrm2_slot, c->st));
-  return QQ_OK;
+int reorth(Arnoldi& A, int idx) {
+  return op_orthonormalize(A.c, A.pb, A.basis(), idx, A.vec(idx), nullptr, A.orth);
 }
 
 int read_H(Arnoldi& A, int ncols, dense::Mat& Hb) {
   std::vector<double> h(2 * (size_t)(A.m + 1) * A.m);
-  QQ_CK(cudaMemcpyAsync(h.data(), A.H.p, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, A.c->st));
+  QQ_CK(cudaMemcpyAsync(h.data(), A.H, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, A.c->st));
   QQ_CK(cudaStreamSynchronize(A.c->st));
   Hb = dense::Mat(ncols + 1, ncols);
   for (int j = 0; j < ncols; ++j)
@@ -173,7 +150,6 @@ int fgmres_fp64(qq_ctx* c, Spinor phi, Spinor x, int m, double resmax, int max_c
   QQ_CK(Z.alloc((size_t)m * A.nel * 16));
   auto zsp = [&](int j) { return Spinor{static_cast<char*>(Z.p) + (size_t)j * A.nel * 16, nullptr, P64}; };
   Tmp tmp(c, P64), r(c, P64);
-  double* nrm2 = c->scal.as<double>() + 8;
   double normnum = 0.0;
   QQ_TRY(true_residual(c, phi, x, r.sp(), tmp.sp(), kappa, &normnum));
   st->mvp += 1;
@@ -191,7 +167,7 @@ int fgmres_fp64(qq_ctx* c, Spinor phi, Spinor x, int m, double resmax, int max_c
     QQ_TRY(A.zeroH());
     for (int j = 0; j < m; ++j) {
       QQ_TRY(M(zsp(j), A.sp(j)));
-      QQ_TRY(arnoldi_step_from(A, j, zsp(j), tmp.sp(), kappa, nrm2));
+      QQ_TRY(arnoldi_step_from(A, j, zsp(j), tmp.sp(), kappa));
       st->itercount += 1;
       st->mvp += 1;
     }
@@ -199,8 +175,8 @@ int fgmres_fp64(qq_ctx* c, Spinor phi, Spinor x, int m, double resmax, int max_c
     QQ_TRY(read_H(A, m, Hb));
     std::vector<dense::cd> y, srv;
     dense::hess_lsq(Hb, cvec, m, y, srv);
-    QQ_TRY(upload_cvec(c, y, A.y.as<double>()));
-    QQ_CK(launch_basis_accum(P64, BasisArgs{Z.p, A.nel, A.nel}, m, A.y.as<double>(), c->g.vh, x, c->st));
+    QQ_TRY(upload_cvec(c, y, A.y));
+    QQ_CK(launch_basis_accum(P64, BasisArgs{Z.p, A.nel, A.nel}, m, A.y, c->g.vh, x, c->st));
     QQ_TRY(true_residual(c, phi, x, r.sp(), tmp.sp(), kappa, &rn));
     st->mvp += 1;
     const double rel = rn / normnum;
@@ -242,7 +218,6 @@ int fgmresdr_fp64(qq_ctx* c, Spinor phi, Spinor x, int m, int k, double resmax, 
   QQ_CK(Z.alloc((size_t)m * A.nel * 16));
   auto zsp = [&](int j) { return Spinor{static_cast<char*>(Z.p) + (size_t)j * A.nel * 16, nullptr, P64}; };
   Tmp tmp(c, P64), r(c, P64);
-  double* nrm2 = c->scal.as<double>() + 8;
   double normnum = 0.0;
   QQ_TRY(true_residual(c, phi, x, r.sp(), tmp.sp(), kappa, &normnum));
   st->mvp += 1;
@@ -260,7 +235,7 @@ int fgmresdr_fp64(qq_ctx* c, Spinor phi, Spinor x, int m, int k, double resmax, 
   for (int cyc = 1; cyc <= max_cycles; ++cyc) {
     for (int j = j0; j < m; ++j) {
       QQ_TRY(M(zsp(j), A.sp(j)));
-      QQ_TRY(arnoldi_step_from(A, j, zsp(j), tmp.sp(), kappa, nrm2));
+      QQ_TRY(arnoldi_step_from(A, j, zsp(j), tmp.sp(), kappa));
       st->itercount += 1;
       st->mvp += 1;
     }
@@ -268,9 +243,9 @@ int fgmresdr_fp64(qq_ctx* c, Spinor phi, Spinor x, int m, int k, double resmax, 
     QQ_TRY(read_H(A, m, Hb));
     std::vector<dense::cd> y, srv;
     dense::hess_lsq(Hb, cvec, m, y, srv);
-    QQ_TRY(upload_cvec(c, y, A.y.as<double>()));
+    QQ_TRY(upload_cvec(c, y, A.y));
     const BasisArgs ZB{Z.p, A.nel, A.nel};
-    QQ_CK(launch_basis_accum(P64, ZB, m, A.y.as<double>(), c->g.vh, x, c->st));
+    QQ_CK(launch_basis_accum(P64, ZB, m, A.y, c->g.vh, x, c->st));
     double rn = 0.0;
     QQ_TRY(true_residual(c, phi, x, r.sp(), tmp.sp(), kappa, &rn));
     st->mvp += 1;
@@ -294,12 +269,12 @@ int fgmresdr_fp64(qq_ctx* c, Spinor phi, Spinor x, int m, int k, double resmax, 
       return QQ_NOT_CONVERGED;
     }
     st->ritz = ritz;
-    QQ_TRY(upload_mat(c, P, A.Pdev.as<double>(), m + 1));
-    QQ_CK(launch_rotate(P64, A.basis(), m + 1, k + 1, A.Pdev.as<double>(), m + 1, c->st));
-    QQ_CK(launch_rotate(P64, ZB, m, k, A.Pdev.as<double>(), m + 1, c->st));
-    QQ_TRY(reorth(A, k, nrm2));
+    QQ_TRY(upload_mat(c, P, A.Pdev, m + 1));
+    QQ_CK(launch_rotate(P64, A.basis(), m + 1, k + 1, A.Pdev, m + 1, c->st));
+    QQ_CK(launch_rotate(P64, ZB, m, k, A.Pdev, m + 1, c->st));
+    QQ_TRY(reorth(A, k));
     QQ_TRY(A.zeroH());
-    QQ_TRY(upload_mat(c, Hk, A.H.as<double>(), m + 1));
+    QQ_TRY(upload_mat(c, Hk, A.H, m + 1));
     std::fill(cvec.begin(), cvec.end(), 0.0);
     for (int i = 0; i <= k; ++i) cvec[i] = cnew[i];
     j0 = k;
@@ -317,7 +292,6 @@ int gmresdr_fp64(qq_ctx* c, Spinor phi, Spinor x, int m, int k, double resmax, i
   Arnoldi A;
   QQ_TRY(A.init(c, P64, m));
   Tmp tmp(c, P64), r(c, P64);
-  double* nrm2 = c->scal.as<double>() + 8;
   double normnum = 0.0;
   QQ_TRY(true_residual(c, phi, x, r.sp(), tmp.sp(), kappa, &normnum));
   st->mvp = 1;
@@ -334,7 +308,7 @@ int gmresdr_fp64(qq_ctx* c, Spinor phi, Spinor x, int m, int k, double resmax, i
   bool restarted = false;
   for (;;) {
     for (int j = j0; j < m; ++j) {
-      QQ_TRY(arnoldi_step(A, j, tmp.sp(), kappa, nrm2));
+      QQ_TRY(arnoldi_step(A, j, tmp.sp(), kappa));
       st->itercount += 1;
       st->mvp += 1;
     }
@@ -342,8 +316,8 @@ int gmresdr_fp64(qq_ctx* c, Spinor phi, Spinor x, int m, int k, double resmax, i
     QQ_TRY(read_H(A, m, Hb));
     std::vector<dense::cd> y, srv;
     dense::hess_lsq(Hb, cvec, m, y, srv);
-    QQ_TRY(upload_cvec(c, y, A.y.as<double>()));
-    QQ_CK(launch_basis_accum(P64, A.basis(), m, A.y.as<double>(), c->g.vh, x, c->st));
+    QQ_TRY(upload_cvec(c, y, A.y));
+    QQ_CK(launch_basis_accum(P64, A.basis(), m, A.y, c->g.vh, x, c->st));
     double rn = 0.0;
     QQ_TRY(true_residual(c, phi, x, r.sp(), tmp.sp(), kappa, &rn));
     st->mvp += 1;
@@ -368,11 +342,11 @@ int gmresdr_fp64(qq_ctx* c, Spinor phi, Spinor x, int m, int k, double resmax, i
       break;
     }
     st->ritz = ritz;
-    QQ_TRY(upload_mat(c, P, A.Pdev.as<double>(), m + 1));
-    QQ_CK(launch_rotate(P64, A.basis(), m + 1, k + 1, A.Pdev.as<double>(), m + 1, c->st));
-    QQ_TRY(reorth(A, k, nrm2));
+    QQ_TRY(upload_mat(c, P, A.Pdev, m + 1));
+    QQ_CK(launch_rotate(P64, A.basis(), m + 1, k + 1, A.Pdev, m + 1, c->st));
+    QQ_TRY(reorth(A, k));
     QQ_TRY(A.zeroH());
-    QQ_TRY(upload_mat(c, Hk, A.H.as<double>(), m + 1));
+    QQ_TRY(upload_mat(c, Hk, A.H, m + 1));
     std::fill(cvec.begin(), cvec.end(), 0.0);
     for (int i = 0; i <= k; ++i) cvec[i] = cnew[i];
     Hk_last = Hk;
@@ -415,7 +389,6 @@ int gmresdrshift_fp64(qq_ctx* c, Spinor b, const std::vector<Spinor>& xs, const 
   A.g5 = true;
   A.g5shift = sigma[0];
   Tmp tmp(c, P64), xb(c, P64), h(c, P64);
-  double* nrm2 = c->scal.as<double>() + 8;
   double* s = c->scal.as<double>();
   double n2 = 0.0;
   QQ_TRY(lin(c, A.sp(0), cimm(1.0), b, cimm(0), Spinor{nullptr, nullptr, P64}, cimm(0),
@@ -436,7 +409,7 @@ int gmresdrshift_fp64(qq_ctx* c, Spinor b, const std::vector<Spinor>& xs, const 
   int j0 = 0, icycle = 1, status = QQ_NOT_CONVERGED;
   for (;;) {
     for (int j = j0; j < m; ++j) {
-      QQ_TRY(arnoldi_step(A, j, tmp.sp(), kappa, nrm2));
+      QQ_TRY(arnoldi_step(A, j, tmp.sp(), kappa));
       st->itercount += 1;
       st->mvp += 1;
     }
@@ -460,9 +433,9 @@ int gmresdrshift_fp64(qq_ctx* c, Spinor b, const std::vector<Spinor>& xs, const 
         d.assign(rhs.begin(), rhs.begin() + m);
         cmult[q] = rhs[m];
       }
-      QQ_TRY(upload_cvec(c, d, A.y.as<double>()));
+      QQ_TRY(upload_cvec(c, d, A.y));
       QQ_TRY(zero_field(c, xb.sp()));
-      QQ_CK(launch_basis_accum(P64, A.basis(), m, A.y.as<double>(), c->g.vh, xb.sp(), c->st));
+      QQ_CK(launch_basis_accum(P64, A.basis(), m, A.y, c->g.vh, xb.sp(), c->st));
       QQ_TRY(lin(c, xs[q], cimm(1.0), xs[q], cimm(1.0), xb.sp()));
       QQ_TRY(op_g5mult(c, h.sp(), xb.sp(), tmp.sp(), 0, kappa, sigma[q]));
       st->mvp += 1;
@@ -493,11 +466,11 @@ int gmresdrshift_fp64(qq_ctx* c, Spinor b, const std::vector<Spinor>& xs, const 
       break;
     }
     st->ritz = ritz;
-    QQ_TRY(upload_mat(c, P, A.Pdev.as<double>(), m + 1));
-    QQ_CK(launch_rotate(P64, A.basis(), m + 1, k + 1, A.Pdev.as<double>(), m + 1, c->st));
-    QQ_TRY(reorth(A, k, nrm2));
+    QQ_TRY(upload_mat(c, P, A.Pdev, m + 1));
+    QQ_CK(launch_rotate(P64, A.basis(), m + 1, k + 1, A.Pdev, m + 1, c->st));
+    QQ_TRY(reorth(A, k));
     QQ_TRY(A.zeroH());
-    QQ_TRY(upload_mat(c, Hk, A.H.as<double>(), m + 1));
+    QQ_TRY(upload_mat(c, Hk, A.H, m + 1));
     std::fill(cvec.begin(), cvec.end(), 0.0);
     for (int i = 0; i <= k; ++i) cvec[i] = cnew[i];
     j0 = k;
@@ -521,7 +494,6 @@ int gmresproj_fp64(qq_ctx* c, Spinor b, Spinor x, int m, int k, double resmax, i
   Arnoldi A;
   QQ_TRY(A.init(c, P64, m));
   Tmp tmp(c, P64), r(c, P64);
-  double* nrm2 = c->scal.as<double>() + 8;
   QQ_TRY(zero_field(c, x));
   double rinit = 0.0;
   QQ_TRY(norm2_host(c, b, &rinit));
@@ -551,8 +523,8 @@ int gmresproj_fp64(qq_ctx* c, Spinor b, Spinor x, int m, int k, double resmax, i
     for (int i = 0; i <= k; ++i) cv[i] = {ch[2 * i], ch[2 * i + 1]};
     std::vector<dense::cd> yp, srvp;
     dense::hess_lsq(defl.Hk, cv, k, yp, srvp);
-    QQ_TRY(upload_cvec(c, yp, A.y.as<double>()));
-    QQ_CK(launch_basis_accum(defl.pb, D, k, A.y.as<double>(), c->g.vh, x, c->st));
+    QQ_TRY(upload_cvec(c, yp, A.y));
+    QQ_CK(launch_basis_accum(defl.pb, D, k, A.y, c->g.vh, x, c->st));
     double beta = 0.0;
     QQ_TRY(true_residual(c, b, x, r.sp(), tmp.sp(), kappa, &beta));
     if (!std::isfinite(beta)) return set_error(QQ_NAN, "NaN residual in gmresproj");
@@ -561,7 +533,7 @@ int gmresproj_fp64(qq_ctx* c, Spinor b, Spinor x, int m, int k, double resmax, i
     cvec[0] = beta;
     QQ_TRY(A.zeroH());
     for (int j = 0; j < m; ++j) {
-      QQ_TRY(arnoldi_step(A, j, tmp.sp(), kappa, nrm2));
+      QQ_TRY(arnoldi_step(A, j, tmp.sp(), kappa));
       st->itercount += 1;
       st->mvp += 1;
     }
@@ -569,8 +541,8 @@ int gmresproj_fp64(qq_ctx* c, Spinor b, Spinor x, int m, int k, double resmax, i
     QQ_TRY(read_H(A, m, Hb));
     std::vector<dense::cd> y, srv;
     dense::hess_lsq(Hb, cvec, m, y, srv);
-    QQ_TRY(upload_cvec(c, y, A.y.as<double>()));
-    QQ_CK(launch_basis_accum(P64, A.basis(), m, A.y.as<double>(), c->g.vh, x, c->st));
+    QQ_TRY(upload_cvec(c, y, A.y));
+    QQ_CK(launch_basis_accum(P64, A.basis(), m, A.y, c->g.vh, x, c->st));
     QQ_TRY(true_residual(c, b, x, r.sp(), tmp.sp(), kappa, &rn));
     st->mvp += 1;
     st->hist.push_back(rn / rinit);
@@ -580,8 +552,8 @@ int gmresproj_fp64(qq_ctx* c, Spinor b, Spinor x, int m, int k, double resmax, i
     if (!std::isfinite(rn)) return set_error(QQ_NAN, "NaN residual in gmresproj");
     // the next projection acts on the least-squares residual V_{m+1} srv
     QQ_TRY(zero_field(c, r.sp()));
-    QQ_TRY(upload_cvec(c, srv, A.y.as<double>()));
-    QQ_CK(launch_basis_accum(P64, A.basis(), m + 1, A.y.as<double>(), c->g.vh, r.sp(), c->st));
+    QQ_TRY(upload_cvec(c, srv, A.y));
+    QQ_CK(launch_basis_accum(P64, A.basis(), m + 1, A.y, c->g.vh, r.sp(), c->st));
     icycle += 1;
   }
   QQ_CK(cudaStreamSynchronize(c->st));
@@ -603,7 +575,6 @@ int gmresdr_mixed(qq_ctx* c, Spinor b, Spinor x, int m, int k, double tol, int m
   Arnoldi A;
   QQ_TRY(A.init(c, P32, m));
   Tmp tmp32(c, P32), tmp64(c, P64), r(c, P64), r32(c, P32);
-  double* nrm2 = c->scal.as<double>() + 8;
   double bn = 0.0;
   QQ_TRY(norm2_host(c, b, &bn));
   bn = std::sqrt(bn);
@@ -626,7 +597,7 @@ int gmresdr_mixed(qq_ctx* c, Spinor b, Spinor x, int m, int k, double tol, int m
   bool restarted = false;
   for (;;) {
     for (int j = j0; j < m; ++j) {
-      QQ_TRY(arnoldi_step(A, j, tmp32.sp(), kappa, nrm2));
+      QQ_TRY(arnoldi_step(A, j, tmp32.sp(), kappa));
       st->itercount += 1;
       st->mvp += 1;
     }
@@ -634,8 +605,8 @@ int gmresdr_mixed(qq_ctx* c, Spinor b, Spinor x, int m, int k, double tol, int m
     QQ_TRY(read_H(A, m, Hb));
     std::vector<dense::cd> y, srv;
     dense::hess_lsq(Hb, cvec, m, y, srv);
-    QQ_TRY(upload_cvec(c, y, A.y.as<double>()));
-    QQ_CK(launch_basis_accum(P32, A.basis(), m, A.y.as<double>(), c->g.vh, x, c->st));
+    QQ_TRY(upload_cvec(c, y, A.y));
+    QQ_CK(launch_basis_accum(P32, A.basis(), m, A.y, c->g.vh, x, c->st));
     QQ_TRY(true_residual(c, b, x, r.sp(), tmp64.sp(), kappa, &rn));
     st->mvp += 1;
     st->true_rel = rn / bn;
@@ -660,9 +631,9 @@ int gmresdr_mixed(qq_ctx* c, Spinor b, Spinor x, int m, int k, double tol, int m
     st->ritz = ritz;
     QQ_TRY(upload_mat(c, P, Pd.as<double>(), m + 1));
     QQ_CK(launch_rotate(P32, A.basis(), m + 1, k + 1, Pd.as<double>(), m + 1, c->st));
-    QQ_TRY(reorth(A, k, nrm2));
+    QQ_TRY(reorth(A, k));
     QQ_TRY(A.zeroH());
-    QQ_TRY(upload_mat(c, Hk, A.H.as<double>(), m + 1));
+    QQ_TRY(upload_mat(c, Hk, A.H, m + 1));
     // c = V_{k+1}^H r with the FP64 residual rounded to the basis precision
     QQ_TRY(lin(c, r32.sp(), cimm(1.0), r.sp()));
     int ng = 0;

@@ -45,6 +45,26 @@ def test_gmresdr_column_counts(pair, m, k):
     assert interior_rel(xe, we, ol.nvhalf) < 1e-8 and interior_rel(xo, wo, ol.nvhalf) < 1e-8
 
 
+@pytest.mark.parametrize("m", [40, 100])
+def test_gmresdr_past_the_krylov_degree(m):
+    """On a unit gauge field the operator has few distinct eigenvalues, so the basis is
+    complete well before m and the rest of the cycle orthogonalises rounding noise: the
+    corrections are as large as the vectors, and the norm is summed directly.  The solve
+    converges in its first cycle with a residual far below its tolerance's 1e-10."""
+    import baylorlqcd_b200 as qq
+
+    lat = qq.Lattice(4, 4, 4, 8, bc=(1, 1, 1, 1))
+    u = np.zeros(lat.gauge_shape)
+    u[:, :, :, : lat.nvhalf, [0, 8, 16]] = 1.0
+    lat.gauge_upload(u)
+    b = random_half(lat.ntotal, lat.nvhalf, 9)
+    x, info = lat.gmresdr(b, lat.new_half(), (m, 8), 1e-10, kappa=(0.11, 0.02))
+    r = b - lat.hdbletm(x, 0, (0.11, 0.02))
+    lat.close()
+    assert info.status == 0 and info.ncycles == 1
+    assert np.linalg.norm(r) <= 1e-10 * np.linalg.norm(b)
+
+
 @pytest.mark.parametrize("nrhs,block,precision", [(1, 1, 32), (5, 3, 32), (33, 32, 32), (5, 8, 16), (3, 2, 64)])
 def test_batch_blocks_share_updates(pair, nrhs, block, precision):
     """Every right-hand side of every block, with the last block short: converged by the
