@@ -26,8 +26,11 @@ NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompil
 # B200 hosts' CPUs) and the plain complex multiply and divide formulas
 # (its values are finite and of modest size: no NaN recovery or range reduction needed)
 # it runs about twice as fast.  Contraction stays off.
-HOST_FLAGS = {"qq_eigen.cu": ["-Xcompiler", "-march=x86-64-v3", "-Xcompiler", "-fcx-limited-range",
-                              "-Xcompiler", "-ffp-contract=off"]}
+# GMRES-DR's restart (harmonic Ritz values of the projected matrix) is the same algebra:
+# 6.9 -> 3.9 ms for m = 60, k = 20.
+_DENSE_FLAGS = ["-Xcompiler", "-march=x86-64-v3", "-Xcompiler", "-fcx-limited-range", "-Xcompiler",
+                "-ffp-contract=off"]
+HOST_FLAGS = {"qq_eigen.cu": _DENSE_FLAGS, "qq_solvers.cu": _DENSE_FLAGS}
 
 
 def _nvcc() -> str:
