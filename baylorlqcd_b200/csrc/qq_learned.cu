@@ -133,23 +133,80 @@ __device__ inline float2 transport_row(const qq::Su3<float>& u, bool back, int a
 
 constexpr int kPtcSites = 64;
 
-// out = layer(w) in for one pair per blockIdx.y; w: [9][COUT][CIN] complex.
-// Bound by the FP32 multiply-adds of the channel mixing; a thread takes one colour of one
-// site, so a layer has three threads per site: enough warps on the small lattices, and no
-// work is repeated but the link's reconstruction.  The weights of one (path, input
-// channel) are read as COUT / 2 16-byte broadcasts.  (With a thread per site an 8 -> 8
-// layer of one pair on 8^3x16 had 64 blocks and took 30 us.  Twenty training steps on two
-// pairs there, 4-8-8-4: 42.2 -> 11.2 ms with this kernel, the weight gradient below and
-// the pairs of a group in one launch.)
+// [path][co][ci] weights -> [path][ci][co] in shared memory: the weights of one (path,
+// input channel) are read as COUT / 2 16-byte broadcasts.
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(kPtcSites * 3) ptc_kernel(NetGeom g, const void* gauge, const float2* __restrict__ in,
-                                                            float2* __restrict__ out, const float2* __restrict__ w) {
-  __shared__ float4 sw[9 * CIN * COUT / 2];  // [path][ci][co]
-  for (int i = threadIdx.y * kPtcSites + threadIdx.x; i < 9 * COUT * CIN; i += 3 * kPtcSites) {
+__device__ inline void ptc_weights(const float2* w, float4* sw, int tid, int threads) {
+  for (int i = tid; i < 9 * COUT * CIN; i += threads) {
     const int ci = i % CIN, co = (i / CIN) % COUT, p = i / (CIN * COUT);
     reinterpret_cast<float2*>(sw)[(p * CIN + ci) * COUT + co] = w[i];
   }
   __syncthreads();
+}
+
+// out = layer(w) in for one pair per blockIdx.y; w: [9][COUT][CIN] complex.  Bound by the
+// FP32 multiply-adds of the channel mixing.  A thread per site: every transport is done
+// once.
+template <int CIN, int COUT>
+__global__ void __launch_bounds__(kNetThreads) ptc_kernel(NetGeom g, const void* gauge, const float2* __restrict__ in,
+                                                          float2* __restrict__ out, const float2* __restrict__ w) {
+  __shared__ float4 sw[9 * CIN * COUT / 2];
+  ptc_weights<CIN, COUT>(w, sw, threadIdx.x, kNetThreads);
+  const int L = blockIdx.x * kNetThreads + threadIdx.x;
+  if (L >= g.V) return;
+  in += (size_t)blockIdx.y * CIN * 3 * g.V;
+  out += (size_t)blockIdx.y * COUT * 3 * g.V;
+  int x[4];
+  lex_coords(g, L, x);
+  float2 acc[COUT][3];
+#pragma unroll
+  for (int co = 0; co < COUT; ++co)
+#pragma unroll
+    for (int a = 0; a < 3; ++a) acc[co][a] = make_float2(0.f, 0.f);
+  for (int p = 0; p < 9; ++p) {
+    const PathSrc ps = path_src(g, x, L, p);
+    if (ps.fac == 0.0f) continue;
+    qq::Su3<float> u;
+    if (p > 0) path_link(g, gauge, x, ps, u);
+    for (int ci = 0; ci < CIN; ++ci) {
+      float2 v[3], t[3];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) v[a] = in[(size_t)(ci * 3 + a) * g.V + ps.L];
+      if (p == 0) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) t[a] = v[a];
+      } else {
+        transport3(u, ps.back, ps.fac, v, t);
+      }
+#pragma unroll
+      for (int co = 0; co < COUT; co += 2) {
+        const float4 wc = sw[((p * CIN + ci) * COUT + co) / 2];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          cmacf(acc[co][a], make_float2(wc.x, wc.y), t[a]);
+          cmacf(acc[co + 1][a], make_float2(wc.z, wc.w), t[a]);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int co = 0; co < COUT; ++co)
+#pragma unroll
+    for (int a = 0; a < 3; ++a) out[(size_t)(co * 3 + a) * g.V + L] = acc[co][a];
+}
+
+// The same with a thread per colour of a site, for lattices whose sites are too few to
+// fill the GPU: three times the threads for one third of the mixing each, the links read
+// and rebuilt by all three.  (8 -> 8 on 8^3x16, one pair: 64 blocks and 30 us with a
+// thread per site.  Twenty training steps on two pairs there, 4-8-8-4: 42.2 -> 11.2 ms with
+// this kernel, the weight gradient below and the pairs of a group in one launch.)
+template <int CIN, int COUT>
+__global__ void __launch_bounds__(kPtcSites * 3) ptc_colour_kernel(NetGeom g, const void* gauge,
+                                                                   const float2* __restrict__ in,
+                                                                   float2* __restrict__ out,
+                                                                   const float2* __restrict__ w) {
+  __shared__ float4 sw[9 * CIN * COUT / 2];
+  ptc_weights<CIN, COUT>(w, sw, threadIdx.y * kPtcSites + threadIdx.x, 3 * kPtcSites);
   const int L = blockIdx.x * kPtcSites + threadIdx.x, a = threadIdx.y;
   if (L >= g.V) return;
   in += (size_t)blockIdx.y * CIN * 3 * g.V;
@@ -385,11 +442,20 @@ __global__ void net_gauss_kernel(int vh, unsigned long long seed, qq::Spinor out
   qq::SpinorIO<qq::P64>::store(out.data, out.norm, vh, s, v);
 }
 
+// A thread per colour up to one block of the thread-per-site kernel on each SM.  Forward
+// pass of 4-8-8-4, thread per site against thread per colour: 8^3x16 100 / 92 us, 8^3x32
+// (16384 sites) 99 / 106 us and 152 / 147 us with 16 channels, 16x16x8x16 124 / 140 us,
+// 12^3x24 141 / 187 us, 16^3x32 267 / 381 us, 24^3x48 1077 / 1745 us.
+constexpr long long kPtcColourSites = 148 * kNetThreads;
+
 template <int CIN, int COUT>
 cudaError_t launch_ptc(const NetGeom& g, const void* gauge, int pairs, const float2* in, float2* out, const float2* w,
                        cudaStream_t st) {
-  ptc_kernel<CIN, COUT><<<dim3((g.V + kPtcSites - 1) / kPtcSites, pairs), dim3(kPtcSites, 3), 0, st>>>(g, gauge, in, out,
-                                                                                                     w);
+  if ((long long)g.V * pairs <= kPtcColourSites)
+    ptc_colour_kernel<CIN, COUT>
+        <<<dim3((g.V + kPtcSites - 1) / kPtcSites, pairs), dim3(kPtcSites, 3), 0, st>>>(g, gauge, in, out, w);
+  else
+    ptc_kernel<CIN, COUT><<<dim3((g.V + kNetThreads - 1) / kNetThreads, pairs), kNetThreads, 0, st>>>(g, gauge, in, out, w);
   return cudaGetLastError();
 }
 // Partials of a weight gradient: about four blocks per SM over the nine paths, and no more

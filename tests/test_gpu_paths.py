@@ -116,6 +116,33 @@ def test_gradient_of_more_pairs_than_a_group(pair, channels):
     assert np.abs(grad - want).max() <= 1e-6 * np.abs(want).max()
 
 
+@pytest.mark.parametrize("dims", [(8, 8, 8, 32), (8, 8, 12, 28)])
+@pytest.mark.parametrize("channels", [(4, 4), (4, 16, 8, 4)])
+def test_layers_on_both_sides_of_the_split(dims, channels):
+    """16384 and 21504 sites: a thread per colour and a thread per site.  FP32 against
+    numpy's FP64 with the bound of the small lattices: a site's sums are as long there."""
+    import baylorlqcd_b200 as qq
+    import netref
+    from qqtest import half_to_lex, random_gauge
+
+    ol = oracle.OracleLattice(*dims, bc=BC)
+    links, u = random_gauge(dims, ol.ntotal, seed=4)
+    net = qq.Net(channels, seed=2)
+    g = random_half(ol.ntotal, ol.nvhalf, seed=7)
+    lat = qq.Lattice(*dims, bc=BC)
+    lat.gauge_upload(u, recon=18)
+    out = net.apply(lat, g)
+    lat.close()
+    w, ch, ws = net.get_weights(), net.channels, []
+    for i in range(len(ch) - 1):
+        n = 9 * ch[i + 1] * ch[i]
+        ws.append(w[:n].reshape(9, ch[i + 1], ch[i]))
+        w = w[n:]
+    net.close()
+    ref = netref.apply(ws, links, half_to_lex(g, dims, 1), BC)
+    assert np.abs(half_to_lex(out, dims, 1) - ref).max() < 2e-5 * np.abs(ref).max()
+
+
 @pytest.mark.parametrize("dims,bc,recon", [((4, 4, 4, 8), (1, 1, 1, -1), 12), ((4, 4, 4, 8), (0, -1, 1, 0), 18),
                                            ((8, 8, 8, 12), (1, -1, 1, -1), 18), ((16, 8, 16, 40), (1, 1, 1, -1), 12)])
 def test_operator_on_reference_arrays(dims, bc, recon):
