@@ -5,6 +5,7 @@
 #include <cmath>
 #include <cstring>
 #include <string>
+#include <vector>
 
 #include "qq_ctx.h"
 
@@ -171,6 +172,36 @@ int hop_tune_key(qq_ctx* c, const HopArgs& a, int prec, int epi) {
   return (((prec * 64 + recon_of(c, prec)) * 64 + a.nrhs) * 4 + epi) * 2 + a.blk;
 }
 
+// The shapes worth timing for a launch.  Each costs four launches and three 256 MiB
+// overwrites, 0.3 ms, at a context's first solve with a block size.  The lists hold every
+// shape that won on eight lattices from 8^4 to 24^3x48, or one within 3% of it (5% for
+// 20 FP32 right-hand sides on 8^3x16).  FP64 blocks keep the whole list: they were not
+// swept.
+//   one right-hand side: 4 threads per site on small lattices (8^4 FP64 10.0 us against
+//     10.7 for the best of the others), 1 or 5 on large FP64 ones (24^3x48 93 us against
+//     131), 304 / 301 on large FP32 ones (50 us against 60), 64 and 128 on 16-bit ones;
+//   FP32: the pipelined kernels up to 11, the copy rings from 6 (12 on 24^3x48: 278 us
+//     against 345); they are the only ones from 12 up;
+//   16 bits: the copy ring from 3 (24^3x48: 108 us against 141) and alone from 4.
+// First solve of a context, the 22 shapes before and these: 12 FP32 right-hand sides on
+// 8^3x16 22.5 -> 14.4 ms and on 16^3x32 69 -> 47, 6 on 12^3x24 26.6 -> 18.9, 1 on 8^4
+// 10.5 -> 9.0, 5 FP16 on 8^3x16 26 -> 23.6; repeated solves as before.
+static std::vector<int> hop_candidates(int prec, int nrhs) {
+  const int M = kShapeMrhs, F = kShapeF2;
+  if (prec == P64) return nrhs == 1 ? std::vector<int>{1, 2, 4, 5, 64} : std::vector<int>{1, 2, 5, 6, 32, 64, 96, 128};
+  if (has_norm(prec)) {
+    if (nrhs == 1) return {1, 2, 4, 64, 128};
+    if (nrhs == 2) return {1, 2, 4, M + 2};
+    if (nrhs == 3) return {1, 2, 4, F + 7, F + 8};
+    return {F + 7, F + 8};
+  }
+  if (nrhs == 1) return {2, 4, 64, F + 1, F + 4};
+  if (nrhs == 2) return {4, F + 1, F + 2, F + 4};
+  if (nrhs <= 5) return {4, 64, F + 1, F + 2, F + 4, F + 6, F + 7};
+  if (nrhs < 12) return {F + 1, F + 4, F + 6, F + 7, F + 8};
+  return {F + 6, F + 7, F + 8, F + 9};
+}
+
 int launch_hop_tuned(qq_ctx* c, const HopArgs& a, int prec, int epi) {
   const int recon = recon_of(c, prec);
   const int key = hop_tune_key(c, a, prec, epi);
@@ -191,22 +222,15 @@ int launch_hop_tuned(qq_ctx* c, const HopArgs& a, int prec, int epi) {
   QQ_CK(tune_flush_buffer(&flush, &flush_bytes));
   int best = 1;
   float best_ms = 1e30f;
-  for (int tps : {1, 2, 5, 6, 32, 64, 96, 128, kShapeMrhs + 2, kShapeMrhs + 3, kShapeMrhs + 4, kShapeF2 + 1,
-                  kShapeF2 + 2, kShapeF2 + 3, kShapeF2 + 4, kShapeF2 + 5, kShapeF2 + 6, kShapeF2 + 7,
-                  kShapeF2 + 8, kShapeF2 + 9, kShapeF2 + 10, kShapeF2 + 11}) {
+  for (int tps : hop_candidates(prec, a.nrhs)) {
     const int per = tps <= 4 ? 128 / tps : tps <= 6 ? 128 : tps;
-    if (a.nrhs > per || ((tps == 5 || tps == 6) && prec != P64)) continue;
-    if (tps >= kShapeF2 + 6) {  // copy ring, every variant (its shared memory pays off from 4 RHS up)
-      const bool ring16 = has_norm(prec) && (tps == kShapeF2 + 7 || tps == kShapeF2 + 8);
-      if ((prec != P32 && !ring16) || a.nrhs < 4) continue;
-    } else if (tps == kShapeF2 + 5) {  // + links staged in shared memory (block fields, nrhs >= 8)
-      if (prec != P32 || !a.blk || a.nrhs < 8) continue;
-    } else if (tps == kShapeF2 + 4) {  // pipelined packed kernel, one RHS per thread
-      if (prec != P32) continue;
-    } else if (tps > kShapeF2) {
+    if (a.nrhs > per) continue;
+    if (tps >= kShapeF2 + 6) {  // copy ring (its shared memory pays off from 4 RHS up, 3 in 16 bits)
+      if (a.nrhs < (has_norm(prec) ? 3 : 4)) continue;
+    } else if (tps > kShapeF2 && tps < kShapeF2 + 4) {
       const int rpt = tps - kShapeF2;
-      if (prec != P32 || a.nrhs % rpt != 0 || (rpt > 1 && !a.blk)) continue;
-    } else if (tps > kShapeMrhs && (!a.blk || prec == P64 || a.nrhs % (tps - kShapeMrhs) != 0)) {
+      if (a.nrhs % rpt != 0 || (rpt > 1 && !a.blk)) continue;
+    } else if (tps > kShapeMrhs && tps < kShapeF2 && (!a.blk || a.nrhs % (tps - kShapeMrhs) != 0)) {
       continue;
     }
     if (launch_hop(a, prec, recon, epi, tps, c->st) != cudaSuccess) {  // warm-up

@@ -82,7 +82,7 @@ def test_batch_blocks_share_updates(pair, nrhs, block, precision):
 
 
 @pytest.mark.parametrize("precision,tol", [(16, 2e-3), (-16, 1.5e-2)])
-@pytest.mark.parametrize("nrhs", [1, 5, 12, 24, 32])
+@pytest.mark.parametrize("nrhs", [1, 3, 5, 12, 24, 32])
 @pytest.mark.parametrize("shape", [307, 308])
 def test_copy_ring_16bit(pair, shape, nrhs, precision, tol):
     """The 16-bit copy ring against the oracle's FP64 Hsingle, with the tolerances of the
@@ -95,6 +95,29 @@ def test_copy_ring_16bit(pair, shape, nrhs, precision, tol):
         for k in {0, nrhs - 1}:
             ref = ol.hsingle(gin[k], idag, gblclr)[..., : ol.nvhalf, :]
             assert np.abs(out[k][..., : ol.nvhalf, :] - ref).max() < tol * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("recon", [12, 18])
+@pytest.mark.parametrize("shape", [1, 2, 4, 5, 64])
+def test_fp64_single(monkeypatch, shape, recon):
+    """The shapes of one FP64 right-hand side, 1280 sites of a parity.  An output
+    component sums 8 hops of 3 products of normal deviates: 1e-13 is 450 rounding errors
+    of the largest."""
+    import baylorlqcd_b200 as qq
+
+    dims = (4, 8, 4, 20)
+    ol = oracle.OracleLattice(*dims, bc=BC)
+    _, u = golden_gauge(dims, ol.ntotal, seed=43, eps=0.3)
+    ol.set_gauge(u)
+    monkeypatch.setenv("QQ_FORCE_TPS", str(shape))
+    lat = qq.Lattice(*dims, bc=BC)
+    lat.gauge_upload(u, recon=recon)
+    gin = random_half(ol.ntotal, ol.nvhalf, 600)
+    for idag, gblclr in ((0, 1), (1, 2)):
+        out = lat.hsingle(gin, idag, gblclr)[..., : ol.nvhalf, :]
+        ref = ol.hsingle(gin, idag, gblclr)[..., : ol.nvhalf, :]
+        assert np.abs(out - ref).max() < 1e-13 * np.abs(ref).max()
+    lat.close()
 
 
 @pytest.mark.parametrize("channels", [(4, 4), (4, 8, 16, 4), (4, 16, 16, 4)])
