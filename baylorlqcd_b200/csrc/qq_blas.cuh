@@ -105,23 +105,17 @@ __global__ void __launch_bounds__(kRedThreads) lincomb_kernel(LinArgs L) {
         o[k] = cadd(o[k], cmulc(c, tt));
       }
     }
-    SpinorIO<PO>::store(L.out.data, L.out.norm, L.vh, s, o);
-    if (L.red >= 1) {
-      // reduce on the stored (rounded) values for FP16 consistency
-      cplx<RO> q[12];
-      if (has_norm(PO))
-        SpinorIO<PO>::load(L.out.data, L.out.norm, L.vh, s, q);
-      else
-        for (int k = 0; k < 12; ++k) q[k] = o[k];
+    SpinorIO<PO>::store_rounded(L.out.data, L.out.norm, L.vh, s, o);
+    if (L.red >= 1) {  // of the stored (rounded) values
 #pragma unroll
-      for (int k = 0; k < 12; ++k) acc[0] += (double)q[k].re * q[k].re + (double)q[k].im * q[k].im;
+      for (int k = 0; k < 12; ++k) acc[0] += (double)o[k].re * o[k].re + (double)o[k].im * o[k].im;
       if (L.red == 2) {
         cplx<typename SpinorIO<PO>::R> wv[12];
         SpinorIO<PO>::load(L.w.data, L.w.norm, L.vh, s, wv);
 #pragma unroll
         for (int k = 0; k < 12; ++k) {
-          acc[1] += (double)wv[k].re * q[k].re + (double)wv[k].im * q[k].im;
-          acc[2] += (double)wv[k].re * q[k].im - (double)wv[k].im * q[k].re;
+          acc[1] += (double)wv[k].re * o[k].re + (double)wv[k].im * o[k].im;
+          acc[2] += (double)wv[k].re * o[k].im - (double)wv[k].im * o[k].re;
         }
       }
     }

@@ -30,6 +30,11 @@ struct SpinorIO<P64> {
 #pragma unroll
     for (int c = 0; c < 12; ++c) f[(size_t)c * vh + s] = make_double2(v[c].re, v[c].im);
   }
+  // Stores v and leaves in it the values that a later load returns.  load() goes through
+  // the read-only path, so a kernel must not load what it has stored itself.
+  __device__ static inline void store_rounded(void* base, float* norm, int vh, int s, cplx<R>* v) {
+    store(base, norm, vh, s, v);
+  }
 };
 
 // FP32 planes hold spin pairs: plane q < 3 is colour q of spins (0, 1), plane q >= 3
@@ -63,6 +68,9 @@ struct SpinorIO<P32> {
       const int a = p32_first(q);
       f[(size_t)q * vh + s] = make_float4(v[a].re, v[a + 3].re, v[a].im, v[a + 3].im);
     }
+  }
+  __device__ static inline void store_rounded(void* base, float* norm, int vh, int s, cplx<R>* v) {
+    store(base, norm, vh, s, v);
   }
 };
 
@@ -110,8 +118,7 @@ struct SpinorIO<P16> {
       }
     }
   }
-  __device__ static inline void store(void* base, float* norm, int vh, int s,
-                                      const cplx<R>* v) {
+  __device__ static inline void store_rounded(void* base, float* norm, int vh, int s, cplx<R>* v) {
     float m = 0.f;
 #pragma unroll
     for (int c = 0; c < 12; ++c) m = fmaxf(m, fmaxf(fabsf(v[c].re), fabsf(v[c].im)));
@@ -122,11 +129,21 @@ struct SpinorIO<P16> {
       int4 t;
       __half2* h = reinterpret_cast<__half2*>(&t);
 #pragma unroll
-      for (int k = 0; k < 4; ++k)
+      for (int k = 0; k < 4; ++k) {
         h[k] = __floats2half2_rn(v[4 * q + k].re * inv, v[4 * q + k].im * inv);
+        const float2 ff = __half22float2(h[k]);
+        v[4 * q + k] = {ff.x * m, ff.y * m};
+      }
       f[(size_t)q * vh + s] = t;
     }
     norm[s] = m;
+  }
+  __device__ static inline void store(void* base, float* norm, int vh, int s,
+                                      const cplx<R>* v) {
+    cplx<R> w[12];
+#pragma unroll
+    for (int c = 0; c < 12; ++c) w[c] = v[c];
+    store_rounded(base, norm, vh, s, w);
   }
 };
 
@@ -152,8 +169,7 @@ struct SpinorIO<PB16> {
       }
     }
   }
-  __device__ static inline void store(void* base, float* norm, int vh, int s,
-                                      const cplx<R>* v) {
+  __device__ static inline void store_rounded(void* base, float* norm, int vh, int s, cplx<R>* v) {
     float m = 0.f;
 #pragma unroll
     for (int c = 0; c < 12; ++c) m = fmaxf(m, fmaxf(fabsf(v[c].re), fabsf(v[c].im)));
@@ -164,11 +180,21 @@ struct SpinorIO<PB16> {
       int4 t;
       __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&t);
 #pragma unroll
-      for (int k = 0; k < 4; ++k)
+      for (int k = 0; k < 4; ++k) {
         h[k] = __floats2bfloat162_rn(v[4 * q + k].re * inv, v[4 * q + k].im * inv);
+        const float2 ff = __bfloat1622float2(h[k]);
+        v[4 * q + k] = {ff.x * m, ff.y * m};
+      }
       f[(size_t)q * vh + s] = t;
     }
     norm[s] = m;
+  }
+  __device__ static inline void store(void* base, float* norm, int vh, int s,
+                                      const cplx<R>* v) {
+    cplx<R> w[12];
+#pragma unroll
+    for (int c = 0; c < 12; ++c) w[c] = v[c];
+    store_rounded(base, norm, vh, s, w);
   }
 };
 

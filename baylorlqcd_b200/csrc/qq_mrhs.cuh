@@ -72,9 +72,9 @@ constexpr double kBreakEps = 1e-12;
 // restart is a reliable update after which the shadow residual becomes the re-inserted
 // FP64 residual (rho = ||r||^2, beta = 0, so the next search direction is r).  The
 // usual shadow residual rhat = r0 is one spin-colour component at one site for a point
-// source: every <rhat, .> is then a single component, which 16-bit storage against the
-// site's norm (or an exact FP32 cancellation) can make exactly zero while the Krylov
-// space is fine; the residual a few iterations on is spread over the lattice.
+// source: every <rhat, .> is then a single component, which a symmetry of the links (or
+// an exact cancellation in low precision) can make exactly zero while the Krylov space
+// is fine; the residual a few iterations on is spread over the lattice.
 constexpr int kMaxRestarts = 8;
 
 enum BiOp : int {
@@ -172,8 +172,7 @@ __global__ void __launch_bounds__(kRedThreads) bicg_block_kernel(BlockBiArgs A) 
         IO::store(A.x.data, A.x.norm, n, s, a);
 #pragma unroll
         for (int q = 0; q < 12; ++q) c[q] = csub(c[q], cmuld(omega, b[q]));
-        IO::store(A.r.data, A.r.norm, n, s, c);
-        if (has_norm(P)) IO::load(A.r.data, A.r.norm, n, s, c);  // reduce what was stored
+        IO::store_rounded(A.r.data, A.r.norm, n, s, c);  // the sums are of what is stored
       }
       // ||r||^2 and, fused, the next iteration's rho' = <rhat, r>
 #pragma unroll

@@ -176,18 +176,15 @@ __global__ void __launch_bounds__(kPendThreads) pend_insert_kernel(PendArgs A, i
     cplx<double> v[12];
     cplx<RB> r[12], h[12];
     SpinorIO<P64>::load(static_cast<const char*>(A.r64) + A.stride * k, nullptr, A.vh, s, v);
+    if (!shadow) SpinorIO<P>::load(A.rhat.data, A.rhat.norm, n, e, h);
 #pragma unroll
     for (int q = 0; q < 12; ++q) r[q] = {(RB)v[q].re, (RB)v[q].im};
-    SpinorIO<P>::store(A.r.data, A.r.norm, n, e, r);
     if (shadow) SpinorIO<P>::store(A.rhat.data, A.rhat.norm, n, e, r);
-    if (mask != PEND_ALL) {
-      // the product of what was stored
-      if (has_norm(P)) SpinorIO<P>::load(A.r.data, A.r.norm, n, e, r);
+    SpinorIO<P>::store_rounded(A.r.data, A.r.norm, n, e, r);
+    if (mask != PEND_ALL) {  // the product of what is stored
       if (shadow) {
 #pragma unroll
         for (int q = 0; q < 12; ++q) h[q] = r[q];
-      } else {
-        SpinorIO<P>::load(A.rhat.data, A.rhat.norm, n, e, h);
       }
 #pragma unroll
       for (int q = 0; q < 12; ++q) {

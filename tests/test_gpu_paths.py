@@ -81,6 +81,20 @@ def test_batch_blocks_share_updates(pair, nrhs, block, precision):
         assert interior_rel(xe[i], we, ol.nvhalf) < 1e-8 and interior_rel(xo[i], wo, ol.nvhalf) < 1e-8
 
 
+@pytest.mark.parametrize("precision", [16, -16])
+@pytest.mark.parametrize("nrhs", [1, 5])
+def test_easy_16bit_solves_need_no_other_precision(pair, precision, nrhs):
+    """Far from critical kappa the 16-bit iteration converges by itself, so long as the
+    products that a reliable update resumes from are those of the residual it stored: no
+    hand-over to FP32, no restart."""
+    ol, lat = pair
+    be = np.stack([random_half(ol.ntotal, ol.nvhalf, 250 + i) for i in range(nrhs)])
+    bo = np.stack([random_half(ol.ntotal, ol.nvhalf, 350 + i) for i in range(nrhs)])
+    _, _, infos = lat.fermprop_batch(be, bo, (0.08, 0.0), precision=precision, tol=1e-10, deflate=0)
+    for i in infos:
+        assert i.status == 0 and i.true_rel <= 1e-10 and i.finished_by == 0 and i.restarts == 0
+
+
 @pytest.mark.parametrize("precision,tol", [(16, 2e-3), (-16, 1.5e-2)])
 @pytest.mark.parametrize("nrhs", [1, 3, 5, 12, 24, 32])
 @pytest.mark.parametrize("shape", [307, 308])
