@@ -294,6 +294,7 @@ extern "C" int qq_average(qq_ctx* c, const double* be, const double* bo, const d
   const size_t nv = c->ref_doubles(), V = 2 * (size_t)c->g.vh;
   const int nt = c->g.n[3], vs = c->g.vh / nt;
   Tmp b0(c, P64), b1(c, P64), y0(c, P64), y1(c, P64), p0(c, P64), p1(c, P64), q0(c, P64), q1(c, P64);
+  QQ_TRY(have({&b0, &b1, &y0, &y1, &p0, &p1, &q0, &q1}));
   const Spinor b[2] = {b0.sp(), b1.sp()}, y[2] = {y0.sp(), y1.sp()};
   const Spinor scratch[2][2] = {{p0.sp(), p1.sp()}, {q0.sp(), q1.sp()}};
   const double* src[4] = {be, bo, xe, xo};

@@ -368,6 +368,7 @@ int bicgstab_block_sync(qq_ctx* c, std::vector<PerRhs*>& rhs, int prec, double t
   QQ_CK(ws_get(c, WS_DSLOTS, sizeof(int) * kMaxBatch, reinterpret_cast<void**>(&ds)));
   unsigned* ctl = reinterpret_cast<unsigned*>(Sd + kScalDoubles);
   Tmp tmp64(c, P64), h(c, P64);
+  QQ_TRY(have({&tmp64, &h}));
   double* s1 = c->scal.as<double>();
   // FP64 residual of x (and of the deflated x) -> slot k of r and rhat
   auto true_res = [&](PerRhs& R, SolveStats& st) -> int {
@@ -772,6 +773,7 @@ int batch_solve(qq_ctx* c, int nrhs, const double* be, const double* bo, const d
   std::vector<double> seconds(nrhs, 0.0);
   std::vector<int> status(nrhs, QQ_OK);
   Tmp fbe(c, P64), fbo(c, P64), h(c, P64), src(c, P64);
+  QQ_TRY(have({&fbe, &fbo, &h, &src}));
   BatchFields F;
   QQ_TRY(F.b.get(c, WS_RHS, nrhs));
   QQ_TRY(F.x.get(c, WS_RHS + 1, nrhs));
@@ -935,6 +937,7 @@ int batch_solve(qq_ctx* c, int nrhs, const double* be, const double* bo, const d
   if (rc != QQ_OK) return rc;
   // odd reconstruction, full-lattice residual, output; one wait for all right-hand sides
   Tmp fxo(c, P64), h2(c, P64);
+  QQ_TRY(have({&fxo, &h2}));
   double* res = nullptr;  // per right-hand side: ||b - M x||^2 and ||b||^2, even then odd
   QQ_CK(ws_get(c, WS_RES, sizeof(double) * 4 * nrhs, reinterpret_cast<void**>(&res)));
   for (int i = 0; i < nrhs; ++i) {
@@ -986,6 +989,7 @@ int tune_batch_shapes(qq_ctx* c, int nrhs, const double kappa[2], const qq_metho
   const int prec = prec_of_code(meth->precision);
   if (prec < 0 || nrhs < 1) return set_error(QQ_BAD_ARG, "bad method or nrhs");
   Tmp a64(c, P64), b64(c, P64), t64(c, P64);
+  QQ_TRY(have({&a64, &b64, &t64}));
   QQ_TRY(zero_field(c, a64.sp()));
   QQ_TRY(op_dbletm(c, b64.sp(), a64.sp(), t64.sp(), 0, kappa));
   QQ_TRY(op_hsingle(c, b64.sp(), a64.sp(), 0, 0));
@@ -1024,6 +1028,7 @@ int hsingle_block(qq_ctx* c, int prec, int nrhs, int shape, double* gout, const 
     QQ_CK(out.norm.alloc(sizeof(float) * vh * nrhs));
   }
   Tmp one(c, P64);
+  QQ_TRY(have({&one}));
   for (int k = 0; k < nrhs; ++k) {
     const double* d = nullptr;
     QQ_TRY(stage_in(c, 1, gin + (size_t)k * nv, nv, &d));

@@ -201,6 +201,7 @@ int qq_hsingle(qq_ctx* c, double* gout, const double* gin, int idag, int gblclr)
     return finish_out(c, 2, gout, dout);
   }
   Tmp in(c, P64), out(c, P64);
+  QQ_TRY(have({&in, &out}));
   QQ_TRY(load_half(c, 1, gin, 1 - pout, in.sp()));
   QQ_TRY(op_hsingle(c, out.sp(), in.sp(), idag, pout));
   return store_half(c, 2, out.sp(), pout, gout);
@@ -222,11 +223,13 @@ int qq_hdbletm(qq_ctx* c, double* he, const double* ge, int idag, const double k
   QQ_TRY(stage_in(c, 1, ge, c->ref_doubles(), &di));
   QQ_TRY(stage_out_begin(c, 2, he, c->ref_doubles(), &dout));
   Tmp tmp(c, P64);
+  QQ_TRY(have({&tmp}));
   if (hop_ref_usable(c, dout, di)) {
     QQ_TRY(op_dbletm_ref(c, dout, di, tmp.sp(), idag, kappa));
     return finish_out(c, 2, he, dout);
   }
   Tmp in(c, P64), out(c, P64);
+  QQ_TRY(have({&in, &out}));
   QQ_TRY(load_half(c, 1, ge, 0, in.sp()));
   QQ_TRY(op_dbletm(c, out.sp(), in.sp(), tmp.sp(), idag, kappa));
   return store_half(c, 2, out.sp(), 0, he);
@@ -242,11 +245,13 @@ int qq_twmshift(qq_ctx* c, double* hwhole, const double* gwhole, int idag, const
   if (!hwhole || !gwhole || !kappa) return set_error(QQ_BAD_ARG, "null argument");
   const size_t nv = c->ref_doubles();
   Tmp ge(c, P64), go(c, P64), he(c, P64), ho(c, P64);
+  QQ_TRY(have({&ge, &go, &he, &ho}));
   QQ_TRY(load_half(c, 1, gwhole, 0, ge.sp()));
   QQ_TRY(load_half(c, 2, gwhole + nv, 1, go.sp()));
   const double fac1 = 1.0 / (2.0 * kappa[1]);
   const double fac2 = 1.0 / (2.0 * kappa[0] * kappa[1]);
   Tmp h(c, P64);
+  QQ_TRY(have({&h}));
   QQ_TRY(op_hsingle(c, h.sp(), go.sp(), idag, 0));
   QQ_CK(launch_spinmix(c->g.vh, ge.sp(), h.sp(), he.sp(), 1.0, -fac2, 0.0, -fac1, P64, c->st));
   QQ_TRY(op_hsingle(c, h.sp(), ge.sp(), idag, 1));
@@ -265,6 +270,7 @@ int qq_gamma5mult(qq_ctx* c, double* he, const double* ge, int idag, const doubl
   if (!he || !ge || !kappa) return set_error(QQ_BAD_ARG, "null argument");
   if (idag != 0 && idag != 1) return set_error(QQ_BAD_ARG, "idag must be 0 or 1");
   Tmp in(c, P64), out(c, P64), tmp(c, P64);
+  QQ_TRY(have({&in, &out, &tmp}));
   QQ_TRY(load_half(c, 1, ge, 0, in.sp()));
   QQ_TRY(op_g5mult(c, out.sp(), in.sp(), tmp.sp(), idag, kappa, 0.0));
   return store_half(c, 2, out.sp(), 0, he);
@@ -284,6 +290,7 @@ int qq_gmresdrshift(qq_ctx* c, const double* b, double* xshift, int nshifts, con
   const double t = 2.0 * kappa[0] * kappa[1];
   if (!(t != 0.0) || !std::isfinite(1.0 / t)) return set_error(QQ_BAD_ARG, "gmresdrshift needs kappa*mu /= 0");
   Tmp fb(c, P64);
+  QQ_TRY(have({&fb}));
   QQ_TRY(load_half(c, 1, b, 0, fb.sp()));
   std::vector<std::unique_ptr<Tmp>> fx, fr;
   std::vector<Spinor> xs, rs;
@@ -310,6 +317,7 @@ int qq_vecdot(qq_ctx* c, const double* a, const double* b, double adb[2]) {
   QQ_TRY(set_device(c));
   if (!a || !b || !adb) return set_error(QQ_BAD_ARG, "null argument");
   Tmp fa(c, P64), fb(c, P64);
+  QQ_TRY(have({&fa, &fb}));
   QQ_TRY(load_half(c, 1, a, 0, fa.sp()));
   QQ_TRY(load_half(c, 2, b, 0, fb.sp()));
   std::complex<double> d;
@@ -350,6 +358,7 @@ int qq_defl_vector(const qq_defl* d, int j, double* v) {
     QQ_TRY(field_to_ref(c, f, 0, o));
   } else {  // a reduced-precision space: through an FP64 temporary
     Tmp t(c, P64);
+    QQ_TRY(have({&t}));
     QQ_TRY(lin(c, t.sp(), cimm(1.0), f));
     QQ_TRY(field_to_ref(c, t.sp(), 0, o));
   }
@@ -365,6 +374,7 @@ int qq_gmresdr(qq_ctx* c, const double* phi, double* x, const int GMRES[2], doub
   QQ_TRY(check_iflag(iflag));
   if (!phi || !x || !GMRES || !kappa) return set_error(QQ_BAD_ARG, "null argument");
   Tmp fphi(c, P64), fx(c, P64);
+  QQ_TRY(have({&fphi, &fx}));
   QQ_TRY(load_half(c, 1, phi, 0, fphi.sp()));
   QQ_TRY(load_half(c, 2, x, 0, fx.sp()));
   Timer t(c);
@@ -386,6 +396,7 @@ int qq_gmresproj(qq_ctx* c, const double* b, double* x, const int GMRES[2], doub
   QQ_TRY(check_iflag(iflag));
   if (!b || !x || !GMRES || !kappa || !defl) return set_error(QQ_BAD_ARG, "null argument");
   Tmp fb(c, P64), fx(c, P64);
+  QQ_TRY(have({&fb, &fx}));
   QQ_TRY(load_half(c, 1, b, 0, fb.sp()));
   Timer t(c);
   SolveStats s;
@@ -416,6 +427,7 @@ int qq_bicgstab(qq_ctx* c, const double* phi, double* x, double resmax, int iter
   QQ_TRY(check_iflag(iflag));
   if (!phi || !x || !kappa) return set_error(QQ_BAD_ARG, "null argument");
   Tmp fphi(c, P64), fx(c, P64);
+  QQ_TRY(have({&fphi, &fx}));
   QQ_TRY(load_half(c, 1, phi, 0, fphi.sp()));
   QQ_TRY(load_half(c, 2, x, 0, fx.sp()));
   Timer t(c);
@@ -440,6 +452,7 @@ int qq_fermprop(qq_ctx* c, const double* be, const double* bo, const double kapp
   if ((inverter == 5 || inverter == 6) && !nGMRES) return set_error(QQ_BAD_ARG, "nGMRES needed");
   if (inverter == 6 && !defl) return set_error(QQ_BAD_ARG, "psc needs a deflation handle");
   Tmp fbe(c, P64), fbo(c, P64), src(c, P64), h(c, P64), fxe(c, P64), fxo(c, P64);
+  QQ_TRY(have({&fbe, &fbo, &src, &h, &fxe, &fxo}));
   QQ_TRY(load_half(c, 1, be, 0, fbe.sp()));
   QQ_TRY(load_half(c, 2, bo, 1, fbo.sp()));
   const double tk = 2.0 * kappa[0] * kappa[1];

@@ -4,6 +4,7 @@
 
 #include <complex>
 #include <functional>
+#include <initializer_list>
 #include <map>
 #include <memory>
 #include <string>
@@ -47,7 +48,10 @@ struct DevBuf {
     p = nullptr;
     bytes = 0;
     cudaError_t e = cudaMalloc(&p, b);
-    if (e == cudaSuccess) bytes = b;
+    if (e == cudaSuccess)
+      bytes = b;
+    else
+      cudaGetLastError();  // reported here, not by the next launch's check
     return e;
   }
   template <class T>
@@ -132,7 +136,8 @@ inline cudaError_t ws_get(qq_ctx* c, int id, size_t bytes, void** p) {
   return e;
 }
 
-// Temporary field from the context pool (returned on scope exit).
+// Temporary field from the context pool (returned on scope exit).  Check have() before
+// the first use: a new field may not fit on the device.
 struct Tmp {
   qq_ctx* c;
   int prec;
@@ -144,6 +149,7 @@ struct Tmp {
   Tmp(const Tmp&) = delete;
   Tmp& operator=(const Tmp&) = delete;
 };
+int have(std::initializer_list<const Tmp*> fields);
 
 // ---- operator and level-1 helpers (qq_ops.cu) ----
 int launch_hop_tuned(qq_ctx* c, const HopArgs& a, int prec, int epi);

@@ -214,6 +214,7 @@ struct EigOp {
   int apply(void* out, const void* in) {
     if (kind == 1) {
       Tmp t(c, P64);
+      QQ_TRY(have({&t}));
       return op_dbletm(c, Spinor{out, nullptr, P64}, Spinor{const_cast<void*>(in), nullptr, P64}, t.sp(), 0,
                        kappa);
     }
@@ -486,6 +487,7 @@ int modes_of_m(qq_ctx* c, qq_eig* E, const Basis& ev, const std::vector<cd>& th,
   // <R, L> = 1, then the residual test on M
   std::vector<int> keep;
   Tmp xe(c, P64), xo(c, P64);
+  QQ_TRY(have({&xe, &xo}));
   for (int e = 0; e < np; ++e) {
     cd rl;
     QQ_TRY(dot_full(c, Rt.v(e), Lt.v(e), hn, &rl));
@@ -560,6 +562,7 @@ int mode_traces(qq_ctx* c, const qq_eig* E, const double* ze, const double* zo, 
   const size_t hn = E->half_nel;
   const int nt = c->g.n[3], n = E->num;
   Tmp zfe(c, P64), zfo(c, P64), g5e(c, P64), g5o(c, P64);
+  QQ_TRY(have({&zfe, &zfo, &g5e, &g5o}));
   QQ_TRY(ref_to_field(c, ze, 0, zfe.sp()));
   QQ_TRY(ref_to_field(c, zo, 1, zfo.sp()));
   T.assign((size_t)n * 18 * nt, 0.0);
@@ -827,6 +830,7 @@ extern "C" int qq_xigenerator(qq_ctx* c, const qq_eig* e, double kappa, double* 
   QQ_CK(cudaSetDevice(c->device));
   const size_t hn = e->half_nel;
   Tmp s1e(c, P64), s1o(c, P64), s2e(c, P64), s2o(c, P64), se(c, P64), so(c, P64), ge(c, P64), go(c, P64);
+  QQ_TRY(have({&s1e, &s1o, &s2e, &s2o, &se, &so, &ge, &go}));
   auto H = [&](const Tmp& out, Spinor in, int pout) { return op_hsingle(c, out.sp(), in, 0, pout); };
   auto axpy = [&](const Tmp& y, double a, const Tmp& x) {
     return lin(c, y.sp(), cimm(1.0), y.sp(), cimm(a), x.sp());
@@ -1000,6 +1004,7 @@ extern "C" int qq_generalaverage(qq_ctx* c, const qq_eig* m, const qq_eig* mp, c
   std::vector<double> NS((size_t)18 * nt);
   {
     Tmp x0(c, P64), x1(c, P64);
+    QQ_TRY(have({&x0, &x1}));
     QQ_TRY(ref_to_field(c, zref + 2 * nv, 0, x0.sp()));
     QQ_TRY(ref_to_field(c, zref + 3 * nv, 1, x1.sp()));
     const Spinor y[2] = {x0.sp(), x1.sp()}, z[2] = {half_of(zx.p, hn, 0), half_of(zx.p, hn, 1)};

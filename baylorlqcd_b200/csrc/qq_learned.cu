@@ -693,6 +693,7 @@ int net_embed_refs(qq_ctx* c, int n, const double* refs, DevBuf& out, std::vecto
   const NetGeom g = net_geom(c);
   const size_t nv = c->ref_doubles();
   Tmp t(c, P64);
+  QQ_TRY(have({&t}));
   if (norm2) norm2->resize(n);
   const int nblk = (c->g.vh + 127) / 128;
   QQ_CK(out.alloc(net_field_bytes(c, 4) * n));
@@ -792,6 +793,7 @@ extern "C" int qq_net_apply(qq_ctx* c, qq_net* net, const double* in, double* ou
   QQ_TRY(net_check(c, net));
   if (!in || !out) return set_error(QQ_BAD_ARG, "null array");
   Tmp a(c, P64), b(c, P64);
+  QQ_TRY(have({&a, &b}));
   const double* d = nullptr;
   QQ_TRY(stage_in(c, 1, in, c->ref_doubles(), &d));
   QQ_TRY(ref_to_field(c, d, 0, a.sp()));
@@ -842,6 +844,7 @@ extern "C" int qq_net_train(qq_ctx* c, qq_net* net, const double kappa[2], int n
     QQ_CK(cudaMemsetAsync(pr->p, 0, net_field_bytes(c, 4) * nsamples, c->st));
   }
   Tmp xf(c, P64), bf(c, P64), tmp(c, P64);
+  QQ_TRY(have({&xf, &bf, &tmp}));
   const int nblk = (c->g.vh + 127) / 128;
   for (int i = 0; i < nsamples; ++i) {
     count_launch();
@@ -920,6 +923,7 @@ static int flexible_solve(qq_ctx* c, qq_net* net, const double* phi, double* x, 
     return set_error(QQ_BAD_ARG, "bad FGMRES arguments");
   if (net) QQ_TRY(net_check(c, net));
   Tmp fphi(c, P64), fx(c, P64);
+  QQ_TRY(have({&fphi, &fx}));
   const size_t nv = c->ref_doubles();
   const double* d = nullptr;
   QQ_TRY(stage_in(c, 1, phi, nv, &d));

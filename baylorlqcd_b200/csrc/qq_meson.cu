@@ -69,6 +69,7 @@ extern "C" int qq_pionrho(qq_ctx* c, const double* xe, const double* xo, int ids
   const int vt = c->g.vh / nt;  // sites of one parity on one time slice
   const size_t nv = c->ref_doubles();
   Tmp f(c, P64);
+  QQ_TRY(have({&f}));
   DevBuf part;
   QQ_CK(part.alloc(sizeof(double) * 3 * nt * 2));
   for (int p = 0; p < 2; ++p) {

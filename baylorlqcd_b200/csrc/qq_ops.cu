@@ -29,16 +29,14 @@ Tmp::Tmp(qq_ctx* c_, int prec_) : c(c_), prec(prec_), idx(-1), f(nullptr) {
       break;
     }
   if (idx < 0) {
-    pool.emplace_back(new Field());
+    std::unique_ptr<Field> nf(new Field());
+    nf->prec = prec;
+    if (nf->data.alloc(field_bytes(prec, c->g.vh)) != cudaSuccess ||
+        (has_norm(prec) && nf->norm.alloc(sizeof(float) * c->g.vh) != cudaSuccess))
+      return;
+    pool.push_back(std::move(nf));
     busy.push_back(false);
     idx = (int)pool.size() - 1;
-    Field* nf = pool.back().get();
-    nf->prec = prec;
-    if (nf->data.alloc(field_bytes(prec, c->g.vh)) != cudaSuccess) {
-      f = nullptr;
-      return;
-    }
-    if (has_norm(prec)) nf->norm.alloc(sizeof(float) * c->g.vh);
   }
   busy[idx] = true;
   f = pool[idx].get();
@@ -46,6 +44,12 @@ Tmp::Tmp(qq_ctx* c_, int prec_) : c(c_), prec(prec_), idx(-1), f(nullptr) {
 
 Tmp::~Tmp() {
   if (idx >= 0) c->pool_busy[prec][idx] = false;
+}
+
+int have(std::initializer_list<const Tmp*> fields) {
+  for (const Tmp* t : fields)
+    if (!t->f) return set_error(QQ_CUDA_ERR, "out of device memory for a temporary field");
+  return QQ_OK;
 }
 
 bool is_device_ptr(const void* p) {
@@ -159,6 +163,7 @@ static cudaError_t tune_flush_buffer(void** p, size_t* bytes) {
   if (!b) {
     e = cudaMalloc(&b, kBytes);
     if (e != cudaSuccess) {
+      cudaGetLastError();
       b = nullptr;
       return e;
     }

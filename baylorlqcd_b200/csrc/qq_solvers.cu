@@ -121,6 +121,7 @@ int upload_mat(qq_ctx* c, const dense::Mat& M, double* dev, int ld) {
 int true_residual(qq_ctx* c, Spinor b, Spinor x, Spinor r, Spinor tmp_odd, const double kappa[2],
                   double* nrm) {
   Tmp h(c, x.prec);
+  QQ_TRY(have({&h}));
   QQ_TRY(op_dbletm(c, h.sp(), x, tmp_odd, 0, kappa));
   double* s = c->scal.as<double>();
   QQ_TRY(lin(c, r, cimm(1.0), b, cimm(-1.0), h.sp(), cimm(0), Spinor{nullptr, nullptr, P64}, s));
@@ -150,6 +151,7 @@ int fgmres_fp64(qq_ctx* c, Spinor phi, Spinor x, int m, double resmax, int max_c
   QQ_CK(Z.alloc((size_t)m * A.nel * 16));
   auto zsp = [&](int j) { return Spinor{static_cast<char*>(Z.p) + (size_t)j * A.nel * 16, nullptr, P64}; };
   Tmp tmp(c, P64), r(c, P64);
+  QQ_TRY(have({&tmp, &r}));
   double normnum = 0.0;
   QQ_TRY(true_residual(c, phi, x, r.sp(), tmp.sp(), kappa, &normnum));
   st->mvp += 1;
@@ -218,6 +220,7 @@ int fgmresdr_fp64(qq_ctx* c, Spinor phi, Spinor x, int m, int k, double resmax, 
   QQ_CK(Z.alloc((size_t)m * A.nel * 16));
   auto zsp = [&](int j) { return Spinor{static_cast<char*>(Z.p) + (size_t)j * A.nel * 16, nullptr, P64}; };
   Tmp tmp(c, P64), r(c, P64);
+  QQ_TRY(have({&tmp, &r}));
   double normnum = 0.0;
   QQ_TRY(true_residual(c, phi, x, r.sp(), tmp.sp(), kappa, &normnum));
   st->mvp += 1;
@@ -292,6 +295,7 @@ int gmresdr_fp64(qq_ctx* c, Spinor phi, Spinor x, int m, int k, double resmax, i
   Arnoldi A;
   QQ_TRY(A.init(c, P64, m));
   Tmp tmp(c, P64), r(c, P64);
+  QQ_TRY(have({&tmp, &r}));
   double normnum = 0.0;
   QQ_TRY(true_residual(c, phi, x, r.sp(), tmp.sp(), kappa, &normnum));
   st->mvp = 1;
@@ -389,6 +393,7 @@ int gmresdrshift_fp64(qq_ctx* c, Spinor b, const std::vector<Spinor>& xs, const 
   A.g5 = true;
   A.g5shift = sigma[0];
   Tmp tmp(c, P64), xb(c, P64), h(c, P64);
+  QQ_TRY(have({&tmp, &xb, &h}));
   double* s = c->scal.as<double>();
   double n2 = 0.0;
   QQ_TRY(lin(c, A.sp(0), cimm(1.0), b, cimm(0), Spinor{nullptr, nullptr, P64}, cimm(0),
@@ -494,6 +499,7 @@ int gmresproj_fp64(qq_ctx* c, Spinor b, Spinor x, int m, int k, double resmax, i
   Arnoldi A;
   QQ_TRY(A.init(c, P64, m));
   Tmp tmp(c, P64), r(c, P64);
+  QQ_TRY(have({&tmp, &r}));
   QQ_TRY(zero_field(c, x));
   double rinit = 0.0;
   QQ_TRY(norm2_host(c, b, &rinit));
@@ -575,6 +581,7 @@ int gmresdr_mixed(qq_ctx* c, Spinor b, Spinor x, int m, int k, double tol, int m
   Arnoldi A;
   QQ_TRY(A.init(c, P32, m));
   Tmp tmp32(c, P32), tmp64(c, P64), r(c, P64), r32(c, P32);
+  QQ_TRY(have({&tmp32, &tmp64, &r, &r32}));
   double bn = 0.0;
   QQ_TRY(norm2_host(c, b, &bn));
   bn = std::sqrt(bn);
@@ -668,6 +675,7 @@ int defl_project(qq_ctx* c, const DeflSpace& d, Spinor b, Spinor x, Spinor r, co
                  double* rn) {
   if (d.k <= 0) return QQ_OK;
   Tmp rl(c, d.pb), tmp64(c, P64);
+  QQ_TRY(have({&rl, &tmp64}));
   DevBuf cd, yd;
   QQ_CK(cd.alloc(sizeof(double) * 2 * 256));
   QQ_CK(yd.alloc(sizeof(double) * 2 * 256));
@@ -699,6 +707,7 @@ int bicgstab_fp64(qq_ctx* c, Spinor phi, Spinor x, double resmax, int itermin, i
                   const double kappa[2], SolveStats* st) {
   using cdd = std::complex<double>;
   Tmp r(c, P64), p(c, P64), rhat(c, P64), v(c, P64), t(c, P64), tmp(c, P64);
+  QQ_TRY(have({&r, &p, &rhat, &v, &t, &tmp}));
   QQ_TRY(op_dbletm(c, t.sp(), x, tmp.sp(), 0, kappa));
   double r0 = 0.0;
   double* s = c->scal.as<double>();

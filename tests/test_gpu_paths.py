@@ -231,3 +231,34 @@ def test_unaligned_device_arrays(pair):
     assert np.abs(got - want).max() <= 1e-13 * np.abs(want).max()
     assert not got[..., ol.nvhalf:, :].any() and not want[..., ol.nvhalf:, :].any()
     assert out[0].item() == 3.0
+
+
+def test_a_full_device_is_an_error():
+    """A call whose fields do not fit on the device reports it, and the next one, with the
+    memory free again, gives the values of a fresh context (the order of a component's
+    sums is the autotuner's choice: 1e-12 of the largest value)."""
+    import torch
+
+    import baylorlqcd_b200 as qq
+
+    dims = (16, 16, 16, 32)  # the eight fields of the call take 100 MB
+
+    def lattice():
+        lat = qq.Lattice(*dims, bc=BC)
+        lat.heatbath(6.0, 2, seed=3)
+        return lat
+
+    lat = lattice()
+    v = [torch.from_numpy(random_half(lat.ntotal, lat.nvhalf, 70 + i)).cuda() for i in range(4)]
+    want = lat.average(*v, 0.15, nsub=4, nmom=1, nop=9)
+    lat.close()
+    lat, held = lattice(), []
+    while (free := torch.cuda.mem_get_info()[0] - (48 << 20)) > 0:
+        held.append(torch.empty(min(free, 1 << 30), dtype=torch.uint8, device="cuda"))
+    with pytest.raises(qq.QQError, match="memory"):
+        lat.average(*v, 0.15, nsub=4, nmom=1, nop=9)
+    held.clear()
+    torch.cuda.empty_cache()
+    got = lat.average(*v, 0.15, nsub=4, nmom=1, nop=9)
+    lat.close()
+    assert np.abs(got - want).max() <= 1e-12 * np.abs(want).max()
