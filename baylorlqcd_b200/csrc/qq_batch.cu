@@ -237,8 +237,7 @@ struct GraphLoop {
   cudaGraphExec_t exec = nullptr;
   cudaStream_t aux = nullptr;  // the context's second stream (kept with the context)
   long long per_iter = 0, per_update = 0;
-  // The launches of a finished run: iters iterations, and at least `updates` runs of the IF
-  // body (the most any right-hand side had; several share a run).
+  // The launches of a finished run: its iterations and runs of the IF body.
   void count(long long iters, long long updates) const { count_launch(per_iter * iters + per_update * updates); }
   ~GraphLoop() {
     if (exec) cudaGraphExecDestroy(exec);
@@ -515,10 +514,9 @@ int bicgstab_block_sync(qq_ctx* c, std::vector<PerRhs*>& rhs, int prec, double t
 // the residual and the re-activation are stream-ordered kernels, the decision a
 // one-thread kernel.  Two drivers share those kernels:
 //  - graph loop (default): one CUDA graph holds the whole solve.  A WHILE conditional
-//    node repeats the iteration; after it one IF node per right-hand side runs that
-//    right-hand side's reliable update when it went pending, and a one-thread kernel
-//    sets the WHILE condition (some right-hand side still moving, fewer than maxiter
-//    iterations).  The host launches the graph once and waits, so a descheduled host
+//    node repeats the iteration; after it an IF node runs the reliable updates of all
+//    right-hand sides that went pending, and a one-thread kernel sets the WHILE
+//    condition (some right-hand side still moving, fewer than maxiter iterations).  The host launches the graph once and waits, so a descheduled host
 //    thread cannot leave the GPU idle, and a pending right-hand side resumes in the
 //    next iteration.  The true-residual history is recorded on the device.
 //  - host loop (when hop profiling is on, or QQ_HOST_LOOP=1): the host queues an
@@ -645,7 +643,6 @@ int bicgstab_block(qq_ctx* c, std::vector<PerRhs*>& rhs, const BatchFields& F, i
     QQ_CK(cudaMemcpyAsync(hits.data(), dhits, sizeof(int) * hits.size(), cudaMemcpyDeviceToHost, c->st));
     QQ_CK(cudaStreamSynchronize(c->st));
     const unsigned* hc = reinterpret_cast<const unsigned*>(hS + kScalDoubles);
-    long long nupd_most = 0;
     const unsigned failed = hc[CTL_FAIL] & all;
     for (int k = 0; k < nb; ++k) {
       SolveStats& st = stats[k];
@@ -658,11 +655,10 @@ int bicgstab_block(qq_ctx* c, std::vector<PerRhs*>& rhs, const BatchFields& F, i
         st.hist_mvp.push_back(1 + 2 * hits[(size_t)k * kHist + j] + j + 1);
       }
       if (nupd > 0) st.true_rel = sk[SC_TRUE];
-      nupd_most = std::max<long long>(nupd_most, nupd);
       if ((failed >> k) & 1u) st.fallback = (int)sk[SC_FAIL];
       st.restarts = (int)sk[SC_NRST];
     }
-    gl.count(hc[CTL_ITER], nupd_most);
+    gl.count(hc[CTL_ITER], hc[CTL_UPDATES]);
     done = hc[CTL_DONE] & ~failed;  // converged
     for (int k = 0; k < nb; ++k) {
       rhs[k]->done = (done >> k) & 1u;

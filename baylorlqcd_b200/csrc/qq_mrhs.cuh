@@ -38,8 +38,8 @@ enum ScalSlot : int {
 // NAN / FAIL / RESTART = right-hand side k iterates / awaits its reliable update or
 // convergence test / is finished (converged or stopped) / is re-inserted / stopped on a
 // non-finite value / stopped without converging (reason in its SC_FAIL) / restarts with
-// its re-inserted residual as the shadow residual; ITER counts the iterations of the
-// graph-driven loop.
+// its re-inserted residual as the shadow residual; ITER and UPDATES count the iterations
+// of the graph-driven loop and those after which it ran the reliable updates.
 enum CtlWord : int {
   CTL_ACTIVE = 0,
   CTL_PENDING = 1,
@@ -49,7 +49,8 @@ enum CtlWord : int {
   CTL_NAN = 5,
   CTL_FAIL = 6,
   CTL_RESTART = 7,
-  kCtlWords = 8
+  CTL_UPDATES = 8,
+  kCtlWords = 9
 };
 
 // Why the batched BiCGStab stopped a right-hand side short of its tolerance; the
@@ -477,8 +478,10 @@ __device__ inline void reliable_resume(unsigned* ctl, int k) {
 }
 
 // IF node of the graph-driven loop: a right-hand side is pending.
-static __global__ void reliable_cond_kernel(const unsigned* ctl, cudaGraphConditionalHandle h) {
-  cudaGraphSetConditional(h, (ctl[CTL_PENDING] & ~ctl[CTL_DONE]) != 0u ? 1u : 0u);
+static __global__ void reliable_cond_kernel(unsigned* ctl, cudaGraphConditionalHandle h) {
+  const unsigned pending = (ctl[CTL_PENDING] & ~ctl[CTL_DONE]) != 0u ? 1u : 0u;
+  ctl[CTL_UPDATES] += pending;
+  cudaGraphSetConditional(h, pending);
 }
 
 // WHILE node: another iteration while a right-hand side of `all` can still move and

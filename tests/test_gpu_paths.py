@@ -95,6 +95,34 @@ def test_easy_16bit_solves_need_no_other_precision(pair, precision, nrhs):
         assert i.status == 0 and i.true_rel <= 1e-10 and i.finished_by == 0 and i.restarts == 0
 
 
+def test_launch_counter_of_the_graph_loop(pair):
+    """The counter knows how often the loop's two bodies ran.  Two equal right-hand sides
+    at several tolerances give the launches of a call, an iteration and an update (three
+    unknowns, five calls); two unlike ones then launch an update for every iteration after
+    which either was updated."""
+    import baylorlqcd_b200 as qq
+
+    ol, lat = pair
+    noise = random_half(ol.ntotal, ol.nvhalf, 31), random_half(ol.ntotal, ol.nvhalf, 32)
+    point = lat.pointsource((1, 1, 1, 1), 1, 1)
+
+    def run(a, b, tol):
+        be, bo = np.stack([a[0], b[0]]), np.stack([a[1], b[1]])
+        n0 = qq.launch_count()
+        _, _, infos = lat.fermprop_batch(be, bo, KAPPA, precision=32, tol=tol, deflate=0)
+        n = qq.launch_count() - n0
+        its = [set((i.hist_mvp - np.arange(len(i.hist_mvp)) - 2) // 2) for i in infos]  # at each update
+        return n, max(i.itercount for i in infos), len(its[0] | its[1]), max(map(len, its))
+
+    run(noise, point, 1e-4)  # tunes the hops
+    same = [run(noise, noise, 10.0 ** -k) for k in (2, 4, 6, 8, 10)]
+    fit = np.array([(1, it, upd) for _, it, upd, _ in same], float)
+    per = np.linalg.lstsq(fit, np.array([n for n, *_ in same], float), rcond=None)[0]
+    assert np.abs(per - np.rint(per)).max() < 1e-6 and np.array_equal(fit @ np.rint(per), [n for n, *_ in same])
+    n, it, upd, most = run(noise, point, 1e-10)
+    assert upd > most and n == np.rint(per) @ (1, it, upd)
+
+
 @pytest.mark.parametrize("precision,tol", [(16, 2e-3), (-16, 1.5e-2)])
 @pytest.mark.parametrize("nrhs", [1, 3, 5, 12, 24, 32])
 @pytest.mark.parametrize("shape", [307, 308])
