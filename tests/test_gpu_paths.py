@@ -1,7 +1,8 @@
 """Edges of the GPU kernels behind the solvers, the network's training and the layout
-conversion: column counts of the one-launch orthonormalisation, blocks of right-hand
-sides that share reliable updates, pairs beyond one group of the network's layers, and
-device arrays that are not 16-byte aligned."""
+conversion: column counts of the three-pass orthonormalisation, blocks of right-hand
+sides that share reliable updates, 16-bit iterations, pairs beyond one group of the
+network's layers, the operator on reference-layout arrays, device arrays that are not
+16-byte aligned, and a device without room."""
 import numpy as np
 import pytest
 
@@ -33,16 +34,82 @@ def interior_rel(a, b, nv):
 
 @pytest.mark.parametrize("m,k", [(2, 1), (9, 3), (17, 6), (66, 20), (127, 40)])
 def test_gmresdr_column_counts(pair, m, k):
-    """Basis sizes on both sides of the kernel's splits: fewer columns than its 16 warps
-    (whose spare warps share the elements), 16 and 17, 64 and 65 (four or eight columns a
-    warp), and the largest.  Both solve to 1e-11, and the operator's condition at this
-    kappa is below 1e2: solutions agree to 1e-8."""
+    """Every column count up to m is orthonormalised, so the sizes cross the kernel's
+    splits at 8, 16, 32 and 64 vectors (lanes in one to eight groups, eight or sixteen
+    columns a lane) and reach the largest.  Both solve to 1e-11, and the operator's
+    condition at this kappa is below 1e2: solutions agree to 1e-8."""
     ol, lat = pair
     be, bo = random_half(ol.ntotal, ol.nvhalf, 5), random_half(ol.ntotal, ol.nvhalf, 6)
     xe, xo, info = lat.fermprop(be, bo, KAPPA, inverter=5, resmax=1e-11, nGMRES=(m, k))
     we, wo, st, _ = ol.fermprop(be, bo, KAPPA, inverter=5, resmax=1e-11, nGMRES=(30, 10))
     assert info.status == 0 and st == 0
     assert interior_rel(xe, we, ol.nvhalf) < 1e-8 and interior_rel(xo, wo, ol.nvhalf) < 1e-8
+
+
+def gram_error(lat, defl):
+    """max |V^H V - 1| of a deflation space's vectors."""
+    import torch
+
+    v = torch.stack([torch.from_numpy(defl.vector(j)[..., : lat.nvhalf, :]).cuda().flatten() for j in range(defl.k + 1)])
+    v = torch.complex(v[:, 0::2], v[:, 1::2])
+    return (v.conj() @ v.T - torch.eye(defl.k + 1, device="cuda")).abs().max().item()
+
+
+@pytest.mark.parametrize("m,k", [(9, 4), (17, 12), (33, 28), (66, 60), (127, 60)])
+def test_restarted_basis_is_orthonormal(m, k):
+    """A restart's vectors are combinations of the whole basis with orthonormal
+    coefficients, so their Gram matrix shows the basis's: classical Gram-Schmidt done
+    twice leaves rounding, m products of length 24576 (below 1e-13 with m <= 127)."""
+    import baylorlqcd_b200 as qq
+
+    lat = qq.Lattice(8, 8, 8, 8, bc=BC)
+    lat.heatbath(6.0, 30, seed=4)
+    b, kappa = random_half(lat.ntotal, lat.nvhalf, 12), (0.156, 0.0)
+    defl = lat.deflation(m, k)
+    x, info = lat.gmresdr(b, lat.new_half(), (m, k), 1e-10, kappa=kappa, defl=defl)
+    assert info.status == 0 and info.ncycles > 1 and defl.k == k
+    r = (b - lat.hdbletm(x, 0, kappa))[..., : lat.nvhalf, :]
+    err = gram_error(lat, defl)
+    defl.close()
+    lat.close()
+    assert np.linalg.norm(r) <= 1e-10 * np.linalg.norm(b) and err < 1e-13
+
+
+@pytest.mark.parametrize("nt", [32, 48])
+def test_large_bases(nt):
+    """65,536 and 98,304 sites of a parity: past 2^19 elements a vector (both in FP64, the
+    second in FP32 too), where the first products of 32 and more vectors are another
+    kernel's.  Each solve is judged by its FP64 residual through the operator."""
+    import baylorlqcd_b200 as qq
+
+    lat = qq.Lattice(16, 16, 16, nt, bc=BC)
+    lat.heatbath(6.0, 20, seed=6)
+    b, kappa = random_half(lat.ntotal, lat.nvhalf, 13), (0.150, 0.01)
+    defl = lat.deflation(66, 30)
+    x, info = lat.gmresdr(b, lat.new_half(), (66, 30), 1e-10, kappa=kappa, defl=defl)
+    assert info.status == 0 and info.ncycles > 1 and gram_error(lat, defl) < 1e-13
+    r = (b - lat.hdbletm(x, 0, kappa))[..., : lat.nvhalf, :]
+    assert np.linalg.norm(r) <= 1e-10 * np.linalg.norm(b)
+    defl.close()
+    half = np.stack([b, random_half(lat.ntotal, lat.nvhalf, 14)])
+    _, _, infos = lat.fermprop_batch(half, half[::-1].copy(), kappa, tol=1e-10)  # FP32 basis, m = 60
+    lat.close()
+    assert all(i.status == 0 and i.true_rel <= 1e-10 and i.finished_by == 0 for i in infos)
+
+
+@pytest.mark.parametrize("m,k", [(9, 3), (17, 6), (40, 12), (60, 20), (100, 40), (127, 40)])
+def test_deflated_batch_column_counts(pair, m, k):
+    """The FP32 basis behind a deflated batch, on both sides of the same splits; 60 and 20
+    are the call's defaults.  Solutions agree with the oracle's as those of the FP64
+    basis do."""
+    ol, lat = pair
+    be = np.stack([random_half(ol.ntotal, ol.nvhalf, 20 + i) for i in range(2)])
+    bo = np.stack([random_half(ol.ntotal, ol.nvhalf, 25 + i) for i in range(2)])
+    xe, xo, infos = lat.fermprop_batch(be, bo, KAPPA, m=m, k=k, tol=1e-10)
+    for i in range(2):
+        assert infos[i].status == 0 and infos[i].true_rel <= 1e-10 and infos[i].finished_by == 0
+        we, wo, st, _ = ol.fermprop(be[i], bo[i], KAPPA, inverter=5, resmax=1e-12, nGMRES=(30, 10))
+        assert interior_rel(xe[i], we, ol.nvhalf) < 1e-8 and interior_rel(xo[i], wo, ol.nvhalf) < 1e-8
 
 
 @pytest.mark.parametrize("m", [40, 100])
@@ -140,7 +207,7 @@ def test_copy_ring_16bit(pair, shape, nrhs, precision, tol):
 
 
 @pytest.mark.parametrize("recon", [12, 18])
-@pytest.mark.parametrize("shape", [1, 2, 4, 5, 64])
+@pytest.mark.parametrize("shape", [1, 2, 4, 5, 6, 64])
 def test_fp64_single(monkeypatch, shape, recon):
     """The shapes of one FP64 right-hand side, 1280 sites of a parity.  An output
     component sums 8 hops of 3 products of normal deviates: 1e-13 is 450 rounding errors
@@ -160,6 +227,28 @@ def test_fp64_single(monkeypatch, shape, recon):
         ref = ol.hsingle(gin, idag, gblclr)[..., : ol.nvhalf, :]
         assert np.abs(out - ref).max() < 1e-13 * np.abs(ref).max()
     lat.close()
+
+
+@pytest.mark.parametrize("recon", [12, 18])
+@pytest.mark.parametrize("shape", [5, 6, 96])
+def test_fp64_blocks(monkeypatch, shape, recon):
+    """The FP64 shapes offered to blocks only by the autotuner's choice, forced on three
+    right-hand sides (42 sites a block of 128 threads, the last one partly empty).  The
+    residual that the solve is judged by is another kernel's."""
+    import baylorlqcd_b200 as qq
+
+    dims = (4, 8, 4, 20)
+    ol = oracle.OracleLattice(*dims, bc=BC)
+    _, u = golden_gauge(dims, ol.ntotal, seed=43, eps=0.3)
+    monkeypatch.setenv("QQ_FORCE_TPS", str(shape))
+    lat = qq.Lattice(*dims, bc=BC)
+    lat.gauge_upload(u, recon=recon)
+    be = np.stack([random_half(ol.ntotal, ol.nvhalf, 610 + i) for i in range(3)])
+    bo = np.stack([random_half(ol.ntotal, ol.nvhalf, 620 + i) for i in range(3)])
+    _, _, infos = lat.fermprop_batch(be, bo, KAPPA, precision=64, tol=1e-12, deflate=0)
+    lat.close()
+    for i in infos:
+        assert i.status == 0 and i.true_rel <= 1e-12 and i.finished_by == 0 and i.restarts == 0
 
 
 @pytest.mark.parametrize("channels", [(4, 4), (4, 8, 16, 4), (4, 16, 16, 4)])
@@ -209,12 +298,14 @@ def test_layers_on_both_sides_of_the_split(dims, channels):
 
 
 @pytest.mark.parametrize("dims,bc,recon", [((4, 4, 4, 8), (1, 1, 1, -1), 12), ((4, 4, 4, 8), (0, -1, 1, 0), 18),
-                                           ((8, 8, 8, 12), (1, -1, 1, -1), 18), ((16, 8, 16, 40), (1, 1, 1, -1), 12)])
+                                           ((8, 8, 8, 12), (1, -1, 1, -1), 18), ((8, 8, 8, 16), (1, 1, 1, -1), 12),
+                                           ((16, 16, 8, 32), (1, 0, 1, -1), 18), ((16, 8, 16, 40), (1, 1, 1, -1), 12),
+                                           ((24, 24, 24, 24), (1, 1, 1, -1), 12), ((24, 24, 24, 24), (1, 1, 1, -1), 18)])
 def test_operator_on_reference_arrays(dims, bc, recon):
     """Hsingle and Hdbletm read and write the reference layout directly: each number of
-    threads per site its rule picks below the largest lattices (1024, 3072 and 40,960 sites
-    of a parity), both link storages, fixed and antiperiodic boundaries; FP64 against the
-    oracle at its other tests' 1e-13."""
+    threads per site its rule picks (256 and 3072 sites of a parity: four; 4096 and 32,768:
+    two; 40,960: one; 165,888: one with capped registers), both link storages, fixed and
+    antiperiodic boundaries; FP64 against the oracle at its other tests' 1e-13."""
     import baylorlqcd_b200 as qq
 
     ol = oracle.OracleLattice(*dims, bc=bc)
