@@ -45,9 +45,12 @@ struct RefHop {
 };
 
 // IN / OUT: the input / the output (and EPI_DBLE's operand) is in the reference layout.
-// Thread layout of hop_kernel for one right-hand side: TPS direction groups per site.
-template <int RECON, int TPS, int EPI, bool IN, bool OUT, int MINB>
-__global__ void __launch_bounds__(128, MINB) hop_ref_kernel(HopArgs a, RefHop f) {
+// Thread layout of hop_kernel for one right-hand side: TPS direction groups per site.  A
+// thread per site has its registers capped for three blocks per SM (uncapped, 226
+// registers and two blocks: 39.1 us against 40.5 for Hdbletm on 24,576 sites of a parity,
+// 55.4 against 43.0 on 40,960, 234 against 199 on 331,776).
+template <int RECON, int TPS, int EPI, bool IN, bool OUT>
+__global__ void __launch_bounds__(128, TPS == 1 ? 3 : 1) hop_ref_kernel(HopArgs a, RefHop f) {
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int s = blockIdx.x * blockDim.x + tx;
   const bool active = s < a.g.vh;
@@ -127,13 +130,11 @@ __global__ void __launch_bounds__(128, MINB) hop_ref_kernel(HopArgs a, RefHop f)
 
 template <int RECON, int EPI, bool IN, bool OUT>
 cudaError_t hop_ref_tps(const HopArgs& a, const RefHop& f, int tps, cudaStream_t st) {
-  const int bx = tps >= 8 ? 128 : 128 / tps;
-  const dim3 grd((a.g.vh + bx - 1) / bx), blk(bx, tps >= 8 ? 1 : tps);
+  const dim3 blk(128 / tps, tps), grd((a.g.vh + blk.x - 1) / blk.x);
   switch (tps) {
-    case 1: hop_ref_kernel<RECON, 1, EPI, IN, OUT, 1><<<grd, blk, 0, st>>>(a, f); break;
-    case 2: hop_ref_kernel<RECON, 2, EPI, IN, OUT, 1><<<grd, blk, 0, st>>>(a, f); break;
-    case 4: hop_ref_kernel<RECON, 4, EPI, IN, OUT, 1><<<grd, blk, 0, st>>>(a, f); break;
-    case 8: hop_ref_kernel<RECON, 1, EPI, IN, OUT, 3><<<grd, blk, 0, st>>>(a, f); break;  // registers for 3 blocks
+    case 1: hop_ref_kernel<RECON, 1, EPI, IN, OUT><<<grd, blk, 0, st>>>(a, f); break;
+    case 2: hop_ref_kernel<RECON, 2, EPI, IN, OUT><<<grd, blk, 0, st>>>(a, f); break;
+    case 4: hop_ref_kernel<RECON, 4, EPI, IN, OUT><<<grd, blk, 0, st>>>(a, f); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
@@ -144,11 +145,14 @@ cudaError_t hop_ref(const HopArgs& a, const RefHop& f, int recon, int tps, cudaS
   return recon == 18 ? hop_ref_tps<18, EPI, IN, OUT>(a, f, tps, st) : hop_ref_tps<12, EPI, IN, OUT>(a, f, tps, st);
 }
 
-// Threads per site: four direction groups while a thread per site leaves warps short of
-// two per scheduler (148 SMs x 4 x 2 x 32 = 37,888 sites: at 8^4 10 us against 15 for a
-// hop, at 12x20x4x28 14 against 16.5), one above; from eight waves of 128-site blocks on,
-// registers capped for three blocks per SM (24^3x48: 92 us against 107).
-int ref_tps(int vh) { return vh < 4096 ? 4 : vh < 37888 ? 2 : vh < 8 * 148 * 128 ? 1 : 8; }
+// Threads per site.  A site's hops in sequence are a chain of loads, so groups of
+// directions side by side win as long as all the blocks run at once: 2 blocks per SM hold
+// 148 * 2 * 128 threads, 9472 sites in four groups and 18,944 in two.  Hdbletm with a cold
+// L2, four / two / one, in us: 2048 sites of a parity 28 / 30 / 36, 8192 31 / 31 / 37,
+// 13,440 40 / 33 / 35, 18,432 42 / 34 / 38, 20,480 48 / 43 / 40, 36,864 61 / 47 / 40,
+// 98,304 128 / 104 / 78.  Two groups start at 4096, where the fields that a caller has
+// just touched are in L2 and they are the faster ones (27 against 28; 6144: 28 / 30).
+int ref_tps(int vh) { return vh < 4096 ? 4 : vh <= 148 * 2 * 64 ? 2 : 1; }
 
 bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
 

@@ -299,13 +299,14 @@ def test_layers_on_both_sides_of_the_split(dims, channels):
 
 @pytest.mark.parametrize("dims,bc,recon", [((4, 4, 4, 8), (1, 1, 1, -1), 12), ((4, 4, 4, 8), (0, -1, 1, 0), 18),
                                            ((8, 8, 8, 12), (1, -1, 1, -1), 18), ((8, 8, 8, 16), (1, 1, 1, -1), 12),
+                                           ((12, 20, 4, 28), (-1, 1, 0, 1), 18),
                                            ((16, 16, 8, 32), (1, 0, 1, -1), 18), ((16, 8, 16, 40), (1, 1, 1, -1), 12),
                                            ((24, 24, 24, 24), (1, 1, 1, -1), 12), ((24, 24, 24, 24), (1, 1, 1, -1), 18)])
 def test_operator_on_reference_arrays(dims, bc, recon):
     """Hsingle and Hdbletm read and write the reference layout directly: each number of
-    threads per site its rule picks (256 and 3072 sites of a parity: four; 4096 and 32,768:
-    two; 40,960: one; 165,888: one with capped registers), both link storages, fixed and
-    antiperiodic boundaries; FP64 against the oracle at its other tests' 1e-13."""
+    threads per site its rule picks (256 and 3072 sites of a parity: four; 4096 and 13,440:
+    two; 32,768 and more: one), both link storages, fixed and antiperiodic boundaries; FP64
+    against the oracle at its other tests' 1e-13."""
     import baylorlqcd_b200 as qq
 
     ol = oracle.OracleLattice(*dims, bc=bc)
