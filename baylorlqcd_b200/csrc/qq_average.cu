@@ -4,7 +4,8 @@
 //
 // Level 1 uses the solution x; level k >= 2 subtracts sub_k = sum_{n=0}^{k+1} kappa^n H^n b,
 // the hopping expansion of the propagator applied to the noise b (H = Hsingle on each
-// half).  For y = x - sub_k, one thread per site evaluates loopops in closed form:
+// half).  For y = x - sub_k, a thread per site and direction evaluates loopops in closed
+// form:
 //   J_mu = conj( y(x+mu)^+ (1 - gamma_mu) U_mu(x)^+ b(x) - y(x)^+ (1 + gamma_mu) U_mu(x) b(x+mu) )
 //   J_5 = conj(y^+ b) (+ 12 on levels k >= 2),  J_{5+mu} = conj(y^+ gamma_mu b),
 // neighbours across the lattice edge times bc(mu), the complex noise kept whole.  Sums

@@ -188,9 +188,10 @@ int block_slot(qq_ctx* c, int prec, int nb, int k, Spinor blockf, Spinor x, int 
 // residual) when the method leaves it at 0.
 constexpr int kStallWindow = 2000;
 // The same for a 16-bit iteration, which the batched FP32 iteration continues when it
-// stops: near critical kappa it stalls at a true residual of ~1e-2 (11 or 8 significant
-// bits), so a shorter window hands it over sooner; where 16-bit converges it gains 10x in
-// far fewer iterations (about 15 at kappa = 0.15).
+// stops.  Where 16 bits pay they gain 10x in fewer iterations (60-250 on 16^3x32 at kappa =
+// 0.1565, 10 at 0.15); where they take more than 400 FP32 is the faster one (24^3x48, kappa =
+// 0.1566, mu = 0.0025, four right-hand sides: FP16 alone 2.32 s in 3000 iterations, handed
+// over 1.79 s in 1640-1780; BF16 alone 5.5 s, handed over 2.0 s).
 constexpr int kStallWindow16 = 400;
 
 // Iteration limit of the batched BiCGStab when the method sets none: 40 iterations per
@@ -841,9 +842,8 @@ int batch_solve(qq_ctx* c, int nrhs, const double* be, const double* bo, const d
       int st = bicgstab_block(c, blk, F, prec, tol_even, 0.1, maxiter, prec == P16 || prec == PB16 ? window16 : window,
                               kappa, defl.k > 0 ? &defl : nullptr,
                               bst);
-      // A 16-bit iteration that stopped short (near critical kappa it stalls at a true
-      // residual of ~1e-2: 11 or 8 significant bits cannot resolve the low modes) is
-      // continued by the batched FP32 BiCGStab from its FP64 solution, before any
+      // A 16-bit iteration that stopped short (near critical kappa on large lattices it gains
+      // too slowly: 11 or 8 significant bits resolve the low modes badly) is continued by the batched FP32 BiCGStab from its FP64 solution, before any
       // right-hand side goes to FP64 GMRES-DR; fallback keeps the 16-bit reason.
       if ((prec == P16 || prec == PB16) && (st == QQ_OK || st == QQ_NOT_CONVERGED)) {
         std::vector<PerRhs*> again;

@@ -256,6 +256,8 @@ static cudaError_t hop_ring16(const HopArgs& a, int epi, cudaStream_t st) {
 // + 9, 10 = copy ring with 2 stages, registers capped for 5 / 6 resident blocks;
 // (+ 7 and + 8 on 16-bit spinors too);
 // + 11 = copy ring with 3 stages and pre-broadcast hop matrices read row by row.
+// The autotuner proposes those that win somewhere (hop_candidates); the rest are there for
+// the callers of qq_hsingle_block and qq_bench_hsingle, which name a shape.
 cudaError_t launch_hop(const HopArgs& a, int sp, int recon, int epi, int tps, cudaStream_t st) {
   count_launch();
   const int maxr = a.blk ? kMaxBatch : kMaxRhs;

@@ -442,10 +442,13 @@ __global__ void net_gauss_kernel(int vh, unsigned long long seed, qq::Spinor out
   qq::SpinorIO<qq::P64>::store(out.data, out.norm, vh, s, v);
 }
 
-// A thread per colour up to one block of the thread-per-site kernel on each SM.  Forward
-// pass of 4-8-8-4, thread per site against thread per colour: 8^3x16 100 / 92 us, 8^3x32
-// (16384 sites) 99 / 106 us and 152 / 147 us with 16 channels, 16x16x8x16 124 / 140 us,
-// 12^3x24 141 / 187 us, 16^3x32 267 / 381 us, 24^3x48 1077 / 1745 us.
+// A thread per colour up to one block of the thread-per-site kernel on each SM.  The line
+// is a compromise between the widths: with 4 or 8 channels the two cross near 10,000 sites,
+// with 16 near 20,000.  Thread per site against thread per colour, a step of training on
+// one pair: 4-8-8-4 346 / 331 us on 8192 sites, 404 / 410 on 12,288, 428 / 447 on 16,384;
+// 4-16-16-4 572 / 530, 667 / 658, 728 / 726 and, on 18,432, 809 / 773; 575 / 604 and 1079 /
+// 1136 on 32,768.  Forward pass of 4-8-8-4: 12^3x24 141 / 187 us, 16^3x32 267 / 381 us,
+// 24^3x48 1077 / 1745 us.
 constexpr long long kPtcColourSites = 148 * kNetThreads;
 
 template <int CIN, int COUT>

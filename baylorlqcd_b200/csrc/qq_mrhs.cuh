@@ -294,7 +294,7 @@ static __global__ void __launch_bounds__(256) partial_fold_kernel(const double* 
 // A right-hand side stops (bicg_fail) when a scalar is not finite, when BiCGStab breaks
 // down (<rhat, r>, <rhat, v>, ||t|| or <t, s> numerically zero), or when `window` > 0
 // iterations have passed since its FP64 true residual last fell 10x (stagnation; the
-// anchor is moved by reliable_decide_kernel).
+// anchor is moved by reliable_decide).
 static __global__ void bicg_scalar_kernel(double* S, const int* slots, const double* partial,
                                           int nblocks, int step, unsigned* ctl, double delta,
                                           double half_tol, int window) {

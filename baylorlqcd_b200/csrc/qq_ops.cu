@@ -188,9 +188,10 @@ int hop_tune_key(qq_ctx* c, const HopArgs& a, int prec, int epi) {
 //   FP32: the pipelined kernels up to 11, the copy rings from 6 (12 on 24^3x48: 278 us
 //     against 345); they are the only ones from 12 up;
 //   16 bits: the copy ring from 3 (24^3x48: 108 us against 141) and alone from 4.
-// First solve of a context, the 22 shapes before and these: 12 FP32 right-hand sides on
-// 8^3x16 22.5 -> 14.4 ms and on 16^3x32 69 -> 47, 6 on 12^3x24 26.6 -> 18.9, 1 on 8^4
-// 10.5 -> 9.0, 5 FP16 on 8^3x16 26 -> 23.6; repeated solves as before.
+// First solve of a context, all 20 shapes against these: 12 FP32 right-hand sides on 8^3x16
+// 22.5 -> 14.4 ms and on 16^3x32 69 -> 47, 6 on 12^3x24 26.6 -> 18.9, 1 on 8^4 10.5 -> 9.0;
+// repeated solves as before.  The other shapes are reached by their code alone
+// (qq_hsingle_block, qq_bench_hsingle).
 static std::vector<int> hop_candidates(int prec, int nrhs) {
   const int M = kShapeMrhs, F = kShapeF2;
   if (prec == P64) return nrhs == 1 ? std::vector<int>{1, 2, 4, 5, 64} : std::vector<int>{1, 2, 5, 6, 32, 64, 96, 128};

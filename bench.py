@@ -168,9 +168,11 @@ def operator_label(mu: float) -> str:
     return "twisted mass mu=%g" % mu if mu else "Wilson"
 
 
-def shape_name(shape: int) -> str:
+def shape_name(shape: int, precision: int = 32) -> str:
     """Kernel behind a hopping-kernel shape code (qq_bench_hsingle)."""
-    if shape in (1, 2, 4):
+    if precision in (16, -16) and shape in (307, 308):
+        return "hop_ring16_kernel"
+    if shape in (1, 2, 4, 5, 6):
         return "hop_kernel"
     if 32 <= shape <= 128:
         return "hop_staged_kernel"
@@ -386,7 +388,7 @@ def run_ours(a, rank, world, local):
     achieved = hop_bytes / (hop_ms * 1e-3) / 1e9 if hop_ms > 0 else 0.0
     gflops = hop_flops / (hop_ms * 1e-3) / 1e9 if hop_ms > 0 else 0.0
     shape = lat.hop_tuned_shape(a.precision, a.rhs_block)
-    traffic = NCU_TRAFFIC.get((shape_name(shape), a.precision, a.rhs_block, dims))
+    traffic = NCU_TRAFFIC.get((shape_name(shape, a.precision), a.precision, a.rhs_block, dims))
 
     # plain FP64 GMRES-DR (the reference method) on the same GPU; its solutions are the
     # FP64 reference solves of the first right-hand sides
@@ -416,9 +418,10 @@ def run_ours(a, rank, world, local):
         "vs_baseline": None,
         "dtype": {-16: "bf16/fp64", 16: "fp16/fp64", 32: "fp32/fp64", 64: "fp64"}[a.precision],
         "data": "synthetic: GPU heatbath configuration (beta=6.0, cold start, %d sweeps), point sources" % a.sweeps,
-        "config": {"workload": "%s %s kappa=%.4f, %d point sources, batched FP%d BiCGStab with FP64 "
+        "config": {"workload": "%s %s kappa=%.4f, %d point sources, batched %s BiCGStab with FP64 "
                                "reliable updates%s, tol %.0e full-lattice FP64; plain = FP64 GMRES-DR(%d,%d)"
-                               % (dims_label(dims), operator_label(a.mu), a.kappa, a.nrhs, a.precision,
+                               % (dims_label(dims), operator_label(a.mu), a.kappa, a.nrhs,
+                                  "BF16" if a.precision == -16 else "FP%d" % a.precision,
                                   " + GMRES-DR deflation" if a.deflate else "", a.tol, a.m, a.k),
                    "lattice": list(dims), "kappa": a.kappa, "mu": a.mu, "nrhs": a.nrhs, "precision": a.precision,
                    "rhs_block": a.rhs_block, "parallelism": "replicas x%d" % world,
@@ -436,7 +439,8 @@ def run_ours(a, rank, world, local):
         "speedup_vs_plain_gmresdr": plain / (spr * world) if spr > 0 else None,
         "e2e": {"value": e2e, "unit": "s/RHS", "h2d_bytes_per_step": 2 * a.nrhs * half_bytes,
                 "d2h_bytes_per_step": 2 * a.nrhs * half_bytes, "steps": ne2e},
-        "roofline": {"bound": "hbm", "kernel": "%s (Dslash, %d-bit, shape %d)" % (shape_name(shape), a.precision, shape),
+        "roofline": {"bound": "hbm", "kernel": "%s (Dslash, %d-bit, shape %d)" % (shape_name(shape, a.precision),
+                                                                                     abs(a.precision), shape),
                      "achieved": achieved, "peak": hbm, "peak_kind": hbm_kind, "unit": "GB/s",
                      "frac": achieved / hbm, "traffic": traffic[0] if traffic else None,
                      "traffic_source": traffic[1] if traffic else None, "launches_measured": nlaunch,
@@ -539,7 +543,7 @@ def run_dslash(a):
     hbm, kind = peaks()
     flops = 1320.0 * lat.nvhalf * 16 * a.nrhs
     lat.close()
-    return {"mode": "dslash", "kernel": "%s (shape %d)" % (shape_name(shape), shape), "lattice": list(dims),
+    return {"mode": "dslash", "kernel": "%s (shape %d)" % (shape_name(shape, a.precision), shape), "lattice": list(dims),
             "precision": a.precision, "nrhs": a.nrhs, "us_per_launch": ms * 1e3, "bytes_per_launch": by,
             "gbs": by / ms / 1e6, "frac": by / ms / 1e6 / hbm, "peak": hbm, "peak_kind": kind,
             "gflops": flops / ms / 1e6, "l2": "512 MiB written between launches"}

@@ -200,9 +200,9 @@ int qq_pointsource(qq_ctx* ctx, double* be, double* bo, const int src[4], int ic
  * with mixed-precision GMRES-DR(m, k) (FP32 Krylov basis and FP32 operator inside
  * FP64 iterative refinement); the others are projected onto it and solved together
  * in blocks with a multi-right-hand-side FP32 (precision = 32) or FP16 (precision =
- * 16) BiCGStab inside FP64 reliable updates.  If that BiCGStab breaks down (a NaN in
- * its recurrences), every unfinished right-hand side of the block is solved again from
- * zero by plain FP64 GMRES-DR(m, k) and reported with fallback = 1.  be/bo/xe/xo: nrhs
+ * 16) BiCGStab inside FP64 reliable updates.  A 16-bit BiCGStab that stops short is
+ * continued by the FP32 one; every right-hand side still unfinished is solved by plain
+ * FP64 GMRES-DR(m, k) (fallback and finished_by below say which).  be/bo/xe/xo: nrhs
  * reference-layout halves each, packed one after the other. */
 typedef struct qq_method {
   int m, k;          /* GMRES-DR(m, k) */

@@ -144,8 +144,8 @@ def test_c2_error_against_fp64_per_precision():
         if prec == 32:
             assert [i.fallback for i in infos] == [0] * 12  # the batched FP32 solve converged on its own
         else:
-            # near critical kappa the 16-bit iteration stalls at ~1e-2 and the batched FP32
-            # iteration finishes from its solution; GMRES-DR is never needed
+            # near critical kappa a 16-bit iteration may gain too slowly; the batched FP32
+            # iteration then finishes from its solution, and GMRES-DR is never needed
             assert all(i.finished_by in (0, 32) for i in infos), [(i.fallback, i.finished_by) for i in infos]
         errs[prec] = max(max(rel(xe[i], xe64[i], nv), rel(xo[i], xo64[i], nv)) for i in range(12))
         assert errs[prec] < 1e-6, (prec, errs[prec])
